@@ -119,7 +119,7 @@ struct Engine {
   FrameCtl* d_ctl = nullptr;
   int* d_cellstart = nullptr;
   unsigned* d_err = nullptr;
-  int* d_epoch = nullptr;   // the sweep epoch, advanced on the device by k_post
+  int* d_epoch = nullptr;   // the sweep epoch, advanced on the device by k_between
   unsigned short* d_roi = nullptr;
   void* d_stage = nullptr;
   size_t stage_bytes = 0;
@@ -136,14 +136,14 @@ struct Engine {
   int* d_done = nullptr;
   int2* d_cellitems = nullptr;
   int* d_stepctr = nullptr;
+  int2* d_after = nullptr;
 
   // scheduling
   cudaStream_t stream = 0;
   cudaStream_t own_stream = nullptr;   // created for graph capture when no stream was set
-  int sweep_grid = 0;
+  Shapes shapes;
   int sweep_ctas_cap = 0;   // 0: the full persistent grid
   int tail_peaks = 8;       // k_tail for frames with at most this many RUNNING peaks (0: never)
-  size_t sweep_smem = 0, cta_smem = 0, warp_smem = 0;
   bool configured = false;
 
   // host mirrors
@@ -182,7 +182,7 @@ struct Engine {
 
   void release_peaks() {
     dfree(d_pk); dfree(d_snap); dfree(d_pkoff); dfree(d_nfit); dfree(d_run); dfree(d_anchor);
-    dfree(d_done); dfree(d_cellitems); dfree(d_stepctr);
+    dfree(d_done); dfree(d_cellitems); dfree(d_stepctr); dfree(d_after);
     cap_total = 0;
   }
   void release() {
@@ -227,6 +227,7 @@ struct Engine {
     s.cell_start = d_cellstart;
     s.cell_items = d_cellitems;
     s.stepctr = d_stepctr;
+    s.after = d_after;
     s.ctl = d_ctl;
     s.err_flag = d_err;
     s.roi_xy = d_roi;
@@ -262,8 +263,7 @@ struct Engine {
     }
     // the FFT PSF and pupil-function models run in the FP64 engine only
     if (cfg.model == M_FFT || cfg.model == M_PUPIL) prec = 64;
-    cudaError_t e = (prec == 32) ? Launch<float>::configure(cfg, &sweep_grid, &sweep_smem, &cta_smem, &warp_smem)
-                                 : Launch<double>::configure(cfg, &sweep_grid, &sweep_smem, &cta_smem, &warp_smem);
+    cudaError_t e = (prec == 32) ? Launch<float>::configure(cfg, &shapes) : Launch<double>::configure(cfg, &shapes);
     if (e != cudaSuccess) {
       set_error("kernel configuration failed (ROI %d, %d pixels): %s", cfg.roi, cfg.nroi,
                 cudaGetErrorString(e));
@@ -344,6 +344,8 @@ struct Engine {
     CK(cudaMalloc(&d_done, c * sizeof(int)));
     CK(cudaMalloc(&d_cellitems, c * sizeof(int2)));
     CK(cudaMalloc(&d_stepctr, c * NCOUNTERS * sizeof(int)));
+    CK(cudaMalloc(&d_after, c * sizeof(int2)));
+    CK(cudaMemset(d_snap, 0, c * sizeof(PeakRec)));   // no attempt's mark
     CK(cudaMemset(d_pk, 0, c * sizeof(PeakRec)));
     CK(cudaMemset(d_done, 0xff, c * sizeof(int)));
     CK(cudaMemset(d_stepctr, 0, c * NCOUNTERS * sizeof(int)));
@@ -398,37 +400,58 @@ struct Engine {
     return 0;
   }
 
-  int grid() const {
-    return (sweep_ctas_cap > 0 && sweep_ctas_cap < sweep_grid) ? sweep_ctas_cap : sweep_grid;
+  // CTAs of a sweep launch.
+  int grid(bool team) const {
+    const int g = team ? shapes.team_grid : shapes.grid;
+    return (sweep_ctas_cap > 0 && sweep_ctas_cap < g) ? sweep_ctas_cap : g;
   }
 
-  int tick() {
+  // Whether a sweep of this many RUNNING peaks (all frames) runs a peak per
+  // team.  A team steps a peak in about half a warp's time, but four warps
+  // together get less done than four warps on four peaks, so teams lose once
+  // the sweep has ready peaks for every warp: about one RUNNING peak in 16 is
+  // ready at a time in frames of 0.5 emitters / um^2 (64 frames of 512 x 512, a
+  // sweep of 214,000 peaks 4.6 ms against 4.2 ms, of 60,000 1.6 against 1.5, of
+  // 22,000 0.42 against 0.45; one frame of 3,355 0.63 against 1.03).
+  bool team_sweep(long long running) const {
+    return shapes.team_grid > 0 && running < 16LL * shapes.grid * shapes.warps;
+  }
+
+  cudaError_t enqueue_sweep(bool team) {
+    return prec == 32 ? Launch<float>::sweep(cfg, fs<float>(), shapes, grid(team), team, stream)
+                      : Launch<double>::sweep(cfg, fs<double>(), shapes, grid(team), team, stream);
+  }
+  // What follows a sweep, or (start) sets the frames up whose fit starts; the
+  // states to poll buffer b (-1: none).
+  cudaError_t enqueue_between(bool start, int b) {
+    FramePoll* p = b < 0 ? nullptr : h_poll[b];
+    unsigned* pe = b < 0 ? nullptr : h_perr + b;
+    return prec == 32 ? Launch<float>::between(cfg, fs<float>(), shapes, start, p, pe, stream)
+                      : Launch<double>::between(cfg, fs<double>(), shapes, start, p, pe, stream);
+  }
+
+  int start_frames() {
+    launches += 1;
+    CK(enqueue_between(true, -1));
+    return 0;
+  }
+
+  int tick(bool team, int b) {
     ticks++;
-    launches += 3;
+    launches += 2;
     cudaEvent_t ta = nullptr, tb = nullptr;
     if (timing && timing_pair(&ta, &tb)) return -1;
-    if (prec == 32) {
-      FrameSet<float> s = fs<float>();
-      CK(Launch<float>::prepare(cfg, s, cta_smem, stream));
-      if (timing) CK(cudaEventRecord(ta, stream));
-      CK(Launch<float>::sweep(cfg, s, grid(), sweep_smem, stream));
-      if (timing) CK(cudaEventRecord(tb, stream));
-      CK(Launch<float>::post(cfg, s, cta_smem, stream));
-    } else {
-      FrameSet<double> s = fs<double>();
-      CK(Launch<double>::prepare(cfg, s, cta_smem, stream));
-      if (timing) CK(cudaEventRecord(ta, stream));
-      CK(Launch<double>::sweep(cfg, s, grid(), sweep_smem, stream));
-      if (timing) CK(cudaEventRecord(tb, stream));
-      CK(Launch<double>::post(cfg, s, cta_smem, stream));
-    }
+    if (timing) CK(cudaEventRecord(ta, stream));
+    CK(enqueue_sweep(team));
+    if (timing) CK(cudaEventRecord(tb, stream));
+    CK(enqueue_between(false, b));
     return 0;
   }
 
   // Run ticks until no frame is pending.  Frames start in SWEEP_PENDING
   // with max_sweeps set by the caller.
   // Two bursts are kept in flight: the next two ticks are queued before the
-  // host reads the frame control blocks of the previous burst, so the
+  // host reads the frames' states after the previous burst, so the
   // device never idles on the host's poll.  Ticks queued after the last
   // frame has finished change nothing (every kernel skips DONE frames).
   // Fits of one or two sweeps (a host-driven sweep loop) keep one burst in
@@ -437,20 +460,31 @@ struct Engine {
     if (ensure_poll_buffers()) return -1;
     bool tail_queued = false;
     const bool ahead = max_sweeps > 2;
-    if (burst_poll(0)) return -1;
+    long long running = 0;   // RUNNING peaks at the latest poll (at most)
+    for (int f = 0; f < F; f++)
+      if (ctl[f].phase == PH_SWEEP_PENDING) running += nfit[f];
+    if (start_frames() || burst_poll(0, team_sweep(running))) return -1;
     int cur = 0;
     for (;;) {
-      if (ahead && burst_poll(1 - cur)) return -1;
+      if (ahead && burst_poll(1 - cur, team_sweep(running))) return -1;
       CK(cudaEventSynchronize(ev_pb[cur]));
       if (h_perr[cur]) {
         CK(cudaStreamSynchronize(stream));
         return check_err_flag() ? -1 : 0;
       }
       bool active = false;
-      for (int f = 0; f < F; f++)
-        if (h_pctl[cur][f].phase != PH_DONE && h_pctl[cur][f].phase != PH_IDLE) active = true;
+      running = 0;
+      for (int f = 0; f < F; f++) {
+        const FramePoll& c = h_poll[cur][f];
+        if (c.phase == PH_DONE || c.phase == PH_IDLE) continue;
+        active = true;
+        running += c.nrun;
+      }
       if (!active) {
-        for (int f = 0; f < F; f++) ctl[f] = h_pctl[cur][f];
+        for (int f = 0; f < F; f++) {
+          ctl[f].sweeps = h_poll[cur][f].sweeps;
+          ctl[f].unconverged = h_poll[cur][f].unconverged;
+        }
         CK(cudaStreamSynchronize(stream));
         return check_err_flag() ? -1 : 0;
       }
@@ -461,28 +495,28 @@ struct Engine {
       if (ahead && tail_peaks > 0 && !tail_queued) {
         bool all = true, any = false;
         for (int f = 0; f < F && all; f++) {
-          const FrameCtl& c = h_pctl[cur][f];
+          const FramePoll& c = h_poll[cur][f];
           if (c.phase == PH_DONE || c.phase == PH_IDLE) continue;
-          if (c.phase == PH_SWEEP_PENDING && c.sweeps > 0 && c.unconverged <= tail_peaks) any = true;
+          if (c.phase == PH_IN_SWEEP && c.sweeps > 0 && c.nrun <= tail_peaks) any = true;
           else all = false;
         }
         if (all && any) {
-          if (prec == 32) CK(Launch<float>::tail(cfg, fs<float>(), tail_peaks, stream));
-          else CK(Launch<double>::tail(cfg, fs<double>(), tail_peaks, stream));
+          if (prec == 32) CK(Launch<float>::tail(cfg, fs<float>(), shapes, tail_peaks, stream));
+          else CK(Launch<double>::tail(cfg, fs<double>(), shapes, tail_peaks, stream));
           launches += 1;
           tail_queued = true;
         }
       }
       if (ahead) {
         cur = 1 - cur;
-      } else if (burst_poll(cur)) {
+      } else if (burst_poll(cur, team_sweep(running))) {
         return -1;
       }
     }
   }
 
   // Pinned buffers and events of the two bursts in flight.
-  FrameCtl* h_pctl[2] = {nullptr, nullptr};
+  FramePoll* h_poll[2] = {nullptr, nullptr};
   unsigned* h_perr = nullptr;
   cudaEvent_t ev_pb[2] = {nullptr, nullptr};
   int pctl_n = 0;
@@ -494,9 +528,9 @@ struct Engine {
     }
     if (pctl_n < F) {
       for (int b = 0; b < 2; b++) {
-        if (h_pctl[b]) cudaFreeHost(h_pctl[b]);
-        h_pctl[b] = nullptr;
-        CK(cudaMallocHost((void**)&h_pctl[b], sizeof(FrameCtl) * F));
+        if (h_poll[b]) cudaFreeHost(h_poll[b]);
+        h_poll[b] = nullptr;
+        CK(cudaMallocHost((void**)&h_poll[b], sizeof(FramePoll) * F));
       }
       pctl_n = F;
     }
@@ -506,9 +540,9 @@ struct Engine {
   void release_poll_buffers() {
     release_graphs();
     for (int b = 0; b < 2; b++) {
-      if (h_pctl[b]) cudaFreeHost(h_pctl[b]);
+      if (h_poll[b]) cudaFreeHost(h_poll[b]);
       if (ev_pb[b]) cudaEventDestroy(ev_pb[b]);
-      h_pctl[b] = nullptr;
+      h_poll[b] = nullptr;
       ev_pb[b] = nullptr;
     }
     if (h_perr) cudaFreeHost(h_perr);
@@ -520,23 +554,23 @@ struct Engine {
   // poll buffer b are captured once and relaunched as one graph while
   // nothing they were captured with changes (model configuration, the frame
   // set's device arrays, launch shapes, poll buffers); anything else
-  // re-captures.  The sweep epoch lives on the device (k_post advances
+  // re-captures.  The sweep epoch lives on the device (k_between advances
   // it), so the captured launches need no per-tick arguments.  With timing
   // on, or SA_CUDA_GRAPHS=0 in the environment, bursts are launched
   // kernel by kernel.
-  cudaGraphExec_t burst_exec[2] = {nullptr, nullptr};
-  std::vector<unsigned char> burst_sig[2];
+  cudaGraphExec_t burst_exec[4] = {nullptr, nullptr, nullptr, nullptr};   // [poll buffer + 2 (teams)]
+  std::vector<unsigned char> burst_sig[4];
   bool use_graphs = !(getenv("SA_CUDA_GRAPHS") && getenv("SA_CUDA_GRAPHS")[0] == '0');
 
   void release_graphs() {
-    for (int b = 0; b < 2; b++) {
+    for (int b = 0; b < 4; b++) {
       if (burst_exec[b]) cudaGraphExecDestroy(burst_exec[b]);
       burst_exec[b] = nullptr;
       burst_sig[b].clear();
     }
   }
 
-  std::vector<unsigned char> burst_signature(int b) const {
+  std::vector<unsigned char> burst_signature(int b, bool team) const {
     std::vector<unsigned char> v;
     auto put = [&v](const void* p, size_t n) {
       const unsigned char* c = static_cast<const unsigned char*>(p);
@@ -550,12 +584,13 @@ struct Engine {
       const FrameSet<double> s = fs<double>();
       put(&s, sizeof(s));
     }
-    const int g = grid();
+    const int g = grid(team);
     put(&g, sizeof(g));
     put(&prec, sizeof(prec));
-    put(&sweep_smem, sizeof(sweep_smem));
-    put(&cta_smem, sizeof(cta_smem));
-    put(&h_pctl[b], sizeof(h_pctl[b]));
+    put(&shapes.smem, sizeof(shapes.smem));
+    put(&shapes.team_smem, sizeof(shapes.team_smem));
+    put(&shapes.cta_smem, sizeof(shapes.cta_smem));
+    put(&h_poll[b], sizeof(h_poll[b]));
     put(&h_perr, sizeof(h_perr));
     put(&ev_pb[b], sizeof(ev_pb[b]));
     put(&stream, sizeof(stream));
@@ -564,27 +599,15 @@ struct Engine {
 
   // The stream work of one burst (captured; no early return, so that the
   // capture is always ended).
-  cudaError_t enqueue_burst(int b) {
+  cudaError_t enqueue_burst(int b, bool team) {
     cudaError_t err = cudaSuccess;
     auto keep = [&err](cudaError_t e) {
       if (err == cudaSuccess) err = e;
     };
     for (int i = 0; i < 2; i++) {
-      if (prec == 32) {
-        const FrameSet<float> s = fs<float>();
-        keep(Launch<float>::prepare(cfg, s, cta_smem, stream));
-        keep(Launch<float>::sweep(cfg, s, grid(), sweep_smem, stream));
-        keep(Launch<float>::post(cfg, s, cta_smem, stream));
-      } else {
-        const FrameSet<double> s = fs<double>();
-        keep(Launch<double>::prepare(cfg, s, cta_smem, stream));
-        keep(Launch<double>::sweep(cfg, s, grid(), sweep_smem, stream));
-        keep(Launch<double>::post(cfg, s, cta_smem, stream));
-      }
+      keep(enqueue_sweep(team));
+      keep(enqueue_between(false, i == 1 ? b : -1));
     }
-    keep(cudaMemcpy2DAsync(h_pctl[b], sizeof(FrameCtl), d_ctl, sizeof(FrameCtl), offsetof(FrameCtl, escaped), F,
-                           cudaMemcpyDeviceToHost, stream));
-    keep(cudaMemcpyAsync(h_perr + b, d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
     // an event record node (a plain record under capture only marks the
     // capture's dependencies and cannot be waited on afterwards)
     keep(cudaEventRecordWithFlags(ev_pb[b], stream, cudaEventRecordExternal));
@@ -593,7 +616,7 @@ struct Engine {
 
   // Launch burst b as a graph; 1 when graphs are not available here (the
   // caller launches kernel by kernel), -1 on error.
-  int burst_graph(int b) {
+  int burst_graph(int b, bool team) {
     if (stream == 0) {
       // the legacy default stream cannot be captured: a blocking stream of
       // our own keeps the same ordering with work on the legacy stream
@@ -604,48 +627,45 @@ struct Engine {
       }
       stream = own_stream;
     }
-    std::vector<unsigned char> sig = burst_signature(b);
-    if (!burst_exec[b] || sig != burst_sig[b]) {
-      if (burst_exec[b]) cudaGraphExecDestroy(burst_exec[b]);
-      burst_exec[b] = nullptr;
+    std::vector<unsigned char> sig = burst_signature(b, team);
+    const int x = b + (team ? 2 : 0);
+    if (!burst_exec[x] || sig != burst_sig[x]) {
+      if (burst_exec[x]) cudaGraphExecDestroy(burst_exec[x]);
+      burst_exec[x] = nullptr;
       cudaGraph_t g = nullptr;
       if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
         use_graphs = false;
         return 1;
       }
-      cudaError_t err = enqueue_burst(b);
+      cudaError_t err = enqueue_burst(b, team);
       const cudaError_t e2 = cudaStreamEndCapture(stream, &g);
       if (err == cudaSuccess) err = e2;
-      if (err == cudaSuccess) err = cudaGraphInstantiate(&burst_exec[b], g, 0);
+      if (err == cudaSuccess) err = cudaGraphInstantiate(&burst_exec[x], g, 0);
       if (g) cudaGraphDestroy(g);
       if (err != cudaSuccess) {
         cudaGetLastError();
-        burst_exec[b] = nullptr;
+        burst_exec[x] = nullptr;
         use_graphs = false;
         return 1;
       }
-      burst_sig[b] = sig;
+      burst_sig[x] = sig;
     }
-    CK(cudaGraphLaunch(burst_exec[b], stream));
+    CK(cudaGraphLaunch(burst_exec[x], stream));
     ticks += 2;
-    launches += 6;
+    launches += 4;
     return 0;
   }
 
-  // Two ticks, then the frame control blocks and the error flag into
+  // Two ticks, then the frames' states and the error flag into
   // pinned buffer b, then its event.
-  int burst_poll(int b) {
+  int burst_poll(int b, bool team) {
     if (use_graphs && !timing) {
-      const int r = burst_graph(b);
+      const int r = burst_graph(b, team);
       if (r <= 0) return r;
     }
     for (int i = 0; i < 2; i++)
-      if (tick()) return -1;
-    // the fields before the device-only lists of every frame's block
-    CK(cudaMemcpy2DAsync(h_pctl[b], sizeof(FrameCtl), d_ctl, sizeof(FrameCtl), offsetof(FrameCtl, escaped), F,
-                         cudaMemcpyDeviceToHost, stream));
-    CK(cudaMemcpyAsync(h_perr + b, d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
+      if (tick(team, i == 1 ? b : -1)) return -1;
     CK(cudaEventRecord(ev_pb[b], stream));
     return 0;
   }
@@ -878,16 +898,16 @@ int insert_peaks(Engine* e, const double* rows, const std::vector<int>& counts, 
   if (e->prec == 32) {
     FrameSet<float> s = e->fs<float>();
     CK(Launch<float>::new_peaks(e->cfg, s, d_rows, ncol, ptype, d_slots, d_frames, n,
-                                ptype != PT_FINDER, e->warp_smem, e->stream));
+                                ptype != PT_FINDER, e->shapes.warp_smem, e->stream));
     if (ptype == PT_FINDER)
-      CK(Launch<float>::new_peaks_finder(e->cfg, s, d_slots, d_ff, d_fn, (int)counts.size(), e->warp_smem, e->stream));
+      CK(Launch<float>::new_peaks_finder(e->cfg, s, d_slots, d_ff, d_fn, (int)counts.size(), e->shapes.warp_smem, e->stream));
     CK(Launch<float>::peak_error(e->cfg, s, d_slots, d_frames, n, e->stream));
   } else {
     FrameSet<double> s = e->fs<double>();
     CK(Launch<double>::new_peaks(e->cfg, s, d_rows, ncol, ptype, d_slots, d_frames, n,
-                                 ptype != PT_FINDER, e->warp_smem, e->stream));
+                                 ptype != PT_FINDER, e->shapes.warp_smem, e->stream));
     if (ptype == PT_FINDER)
-      CK(Launch<double>::new_peaks_finder(e->cfg, s, d_slots, d_ff, d_fn, (int)counts.size(), e->warp_smem, e->stream));
+      CK(Launch<double>::new_peaks_finder(e->cfg, s, d_slots, d_ff, d_fn, (int)counts.size(), e->shapes.warp_smem, e->stream));
     CK(Launch<double>::peak_error(e->cfg, s, d_slots, d_frames, n, e->stream));
   }
   e->launches += (ptype == PT_FINDER) ? 3 : 2;
@@ -1000,10 +1020,10 @@ int props_device(Engine* e, int frame0, const std::vector<int>& counts, double* 
   CK(cudaMemcpyAsync(d_frames, frames.data(), ib, cudaMemcpyHostToDevice, e->stream));
   if (e->prec == 32)
     CK(Launch<float>::peak_props(e->cfg, e->fs<float>(), d_slots, d_frames, n, d_sum, d_fg, d_bg,
-                                 jac ? d_jac : nullptr, e->warp_smem, e->stream));
+                                 jac ? d_jac : nullptr, e->shapes.warp_smem, e->stream));
   else
     CK(Launch<double>::peak_props(e->cfg, e->fs<double>(), d_slots, d_frames, n, d_sum, d_fg, d_bg,
-                                  jac ? d_jac : nullptr, e->warp_smem, e->stream));
+                                  jac ? d_jac : nullptr, e->shapes.warp_smem, e->stream));
   if (sum) CK(cudaMemcpyAsync(sum, d_sum, db, cudaMemcpyDeviceToHost, e->stream));
   if (fg) CK(cudaMemcpyAsync(fg, d_fg, db, cudaMemcpyDeviceToHost, e->stream));
   if (bg) CK(cudaMemcpyAsync(bg, d_bg, db, cudaMemcpyDeviceToHost, e->stream));
@@ -1497,8 +1517,8 @@ void mFitSetPeakStatus(saFitData* h, int32_t* status) {
   cudaMemcpyAsync(d_frames, frames.data(), ib, cudaMemcpyHostToDevice, e->stream);
   cudaMemcpyAsync(d_status, status, ib, cudaMemcpyHostToDevice, e->stream);
   cudaError_t err = (e->prec == 32)
-                        ? Launch<float>::set_status(e->cfg, e->fs<float>(), d_slots, d_frames, d_status, n, e->warp_smem, e->stream)
-                        : Launch<double>::set_status(e->cfg, e->fs<double>(), d_slots, d_frames, d_status, n, e->warp_smem, e->stream);
+                        ? Launch<float>::set_status(e->cfg, e->fs<float>(), d_slots, d_frames, d_status, n, e->shapes.warp_smem, e->stream)
+                        : Launch<double>::set_status(e->cfg, e->fs<double>(), d_slots, d_frames, d_status, n, e->shapes.warp_smem, e->stream);
   if (err != cudaSuccess) set_error("set status: %s", cudaGetErrorString(err));
   cudaStreamSynchronize(e->stream);
   e->host_valid = false;
@@ -1596,7 +1616,7 @@ int saSetSchedule(saFitData* h, int dil_late, int dil_switch) {
 int saGetSweepGrid(saFitData* h) {
   Engine* e = E(h);
   if (!e || !e->configured) return -1;
-  return e->sweep_grid;
+  return e->shapes.grid;
 }
 
 int saSetTailPeaks(saFitData* h, int peaks) {
@@ -1813,8 +1833,8 @@ int saSetPeakStatusBatch(saFitData* h, const int32_t* status) {
   CK(cudaMemcpyAsync(d_frames, frames.data(), ib, cudaMemcpyHostToDevice, e->stream));
   CK(cudaMemcpyAsync(d_status, status, ib, cudaMemcpyHostToDevice, e->stream));
   CK((e->prec == 32)
-         ? Launch<float>::set_status(e->cfg, e->fs<float>(), d_slots, d_frames, d_status, n, e->warp_smem, e->stream)
-         : Launch<double>::set_status(e->cfg, e->fs<double>(), d_slots, d_frames, d_status, n, e->warp_smem,
+         ? Launch<float>::set_status(e->cfg, e->fs<float>(), d_slots, d_frames, d_status, n, e->shapes.warp_smem, e->stream)
+         : Launch<double>::set_status(e->cfg, e->fs<double>(), d_slots, d_frames, d_status, n, e->shapes.warp_smem,
                                       e->stream));
   e->launches += 1;
   CK(cudaStreamSynchronize(e->stream));
@@ -1990,12 +2010,21 @@ int saSlotLoad(saFitData* h, int slot, const void* image, const void* background
     set_error("saSlotLoad: %d peaks, slot capacity %d", n_peaks, e->cap_f[slot]);
     return -1;
   }
-  // the slot is idle while its frame and peaks are replaced
+  // The slot is idle while its frame and peaks are replaced.  The attempt
+  // count goes on: the start records of earlier fits carry it as their mark.
   FrameCtl c;
   memset(&c, 0, sizeof(c));
   c.phase = PH_IDLE;
   c.escaped_min = INT_MAX;
-  CK(cudaMemcpyAsync(e->d_ctl + slot, &c, sizeof(c), cudaMemcpyHostToDevice, e->stream));
+  auto put_ctl = [&]() {
+    char* d = reinterpret_cast<char*>(e->d_ctl + slot);
+    const char* h = reinterpret_cast<const char*>(&c);
+    const size_t at = offsetof(FrameCtl, attempt), to = at + sizeof(c.attempt);
+    CK(cudaMemcpyAsync(d, h, at, cudaMemcpyHostToDevice, e->stream));
+    CK(cudaMemcpyAsync(d + to, h + to, sizeof(c) - to, cudaMemcpyHostToDevice, e->stream));
+    return 0;
+  };
+  if (put_ctl()) return -1;
   const size_t bytes = (size_t)e->npix * (bits / 8);
   if (e->stage(2 * bytes)) return -1;
   char* st = (char*)e->d_stage;
@@ -2016,8 +2045,7 @@ int saSlotLoad(saFitData* h, int slot, const void* image, const void* background
   if (insert_peaks(e, peaks, counts, pt)) return -1;
   c.phase = PH_SWEEP_PENDING;
   c.max_sweeps = max_iterations + 1;   // dao_fit_c.py:340-346
-  CK(cudaMemcpyAsync(e->d_ctl + slot, &c, sizeof(c), cudaMemcpyHostToDevice, e->stream));
-  return 0;
+  return put_ctl();
 }
 
 int saSlotLaunch(saFitData* h, int n_ticks) {
@@ -2030,8 +2058,10 @@ int saSlotLaunch(saFitData* h, int n_ticks) {
     e->h_ctl_n = e->F;
   }
   if (!e->ev_poll) CK(cudaEventCreateWithFlags(&e->ev_poll, cudaEventDisableTiming));
+  if (e->start_frames()) return -1;
+  const bool team = e->team_sweep(0);   // a serving grid is small: its lanes share the GPU
   for (int i = 0; i < n_ticks; i++)
-    if (e->tick()) return -1;
+    if (e->tick(team, -1)) return -1;
   CK(cudaMemcpy2DAsync(e->h_ctl, sizeof(FrameCtl), e->d_ctl, sizeof(FrameCtl), offsetof(FrameCtl, escaped), e->F,
                        cudaMemcpyDeviceToHost, e->stream));
   CK(cudaEventRecord(e->ev_poll, e->stream));

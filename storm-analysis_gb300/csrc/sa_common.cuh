@@ -47,7 +47,7 @@ constexpr double FX_INV = 1.0 / 68719476736.0;
 enum { PT_FINDER = 0, PT_TESTING = 1, PT_TEXT = 2 };
 
 // Frame phases of the device-side doFit state machine.
-enum { PH_IDLE = 0, PH_SWEEP_PENDING = 1, PH_IN_SWEEP = 2, PH_RERUN_PENDING = 3, PH_DONE = 4 };
+enum { PH_IDLE = 0, PH_SWEEP_PENDING = 1, PH_IN_SWEEP = 2, PH_DONE = 4 };
 
 constexpr int MAX_BARRIERS = 256;     // per frame; beyond this the frame runs in index order
 constexpr int MAX_ESCAPES = 128;      // per sweep attempt; beyond this likewise
@@ -108,10 +108,19 @@ struct FrameCtl {
   int reruns_total;      // sweep attempts beyond the first, all sweeps
   int barriers_total;    // escaped peaks made barriers, all sweeps
   int dil;               // footprint dilation of the current sweep
+  int attempt;           // sweep attempts so far, all fits: marks the start records in snap
   long long ctr[NCOUNTERS];
   // device-only lists (the host's polls copy the fields above them)
   int escaped[MAX_ESCAPES];
   int barrier[MAX_BARRIERS];   // ascending
+};
+
+enum { AFTER_RUNNING = 1, AFTER_MOVES = 2 };   // still RUNNING; and to be recentered
+
+// A frame's state as the host polls it: k_between writes it to pinned host
+// memory (two copy nodes per poll took as long as a small sweep).
+struct FramePoll {
+  int phase, sweeps, unconverged, nrun;
 };
 
 // Device pointers of a frame set.  T is the pixel arithmetic type.
@@ -136,10 +145,11 @@ struct FrameSet {
   int* run;              // run list: local peak index per run rank
   unsigned* anchor0;     // packed (xi | yi << 16) per run rank at sweep start
   int* done;             // epoch per run rank
-  int* epoch;            // epoch of the current tick (one int; k_post advances it)
+  int* epoch;            // epoch of the current tick (one int; k_between advances it)
   int* cell_start;       // [F][gx*gy+1]
   int2* cell_items;      // run ranks grouped by cell, each with its packed anchor
   int* stepctr;          // [peaks][NCOUNTERS] counters of the latest step of each peak
+  int2* after;           // per run rank, what its step left: packed anchor, AFTER_* flags
   FrameCtl* ctl;
   unsigned* err_flag;    // bit 0: wait timeout, bit 1: ROI too large
   const unsigned short* roi_xy;  // packed (rx | ry << 8)

@@ -317,6 +317,12 @@ __device__ __forceinline__ long long fx_round(float y) {
 __device__ __forceinline__ long long fixed_from_ff(ff a) {
   return fx_round(__fmul_rn(a.h, 68719476736.0f)) + fx_round(__fmul_rn(a.l, 68719476736.0f));
 }
+// The same out of line, for the team step: it runs through its code once, and
+// fetching the code is much of its time (warps with no instruction to issue
+// were the largest stall), so what several phases use is kept once.  With this
+// and g32_table_axis out of line the 64-frame batch's first sweep took 4.6 ms
+// instead of 5.2.
+static __device__ __noinline__ long long fixed_from_ff_call(ff a) { return fixed_from_ff(a); }
 
 __device__ __forceinline__ ff two_prod(float a, float b) {
   const float p = __fmul_rn(a, b);
@@ -409,6 +415,33 @@ __device__ __forceinline__ ff warp_transpose_sum32_ff(float (&v)[32], int lane) 
     }
   }
   return w[0];
+}
+
+// Reduce 16 float values held by every lane in float-float additions:
+// afterwards lane L holds the warp total of value L >> 1 (partners 16, 8,
+// 4, 2, 1 lanes away: no rounding beyond the inputs' to ~1e-14).
+__device__ __forceinline__ ff warp_reduce16_to_ff(float (&v)[16], int lane) {
+  ff w[8];
+  {
+    const bool up = (lane & 16) != 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const float send = up ? v[i] : v[i + 8];
+      const float keep = up ? v[i + 8] : v[i];
+      w[i] = two_sum(keep, __shfl_xor_sync(0xffffffffu, send, 16));
+    }
+  }
+#pragma unroll
+  for (int h = 8, m = 4; h >= 2; h >>= 1, m >>= 1) {
+    const bool up = (lane & h) != 0;
+#pragma unroll
+    for (int i = 0; i < m; i++) {
+      const ff send = up ? w[i] : w[i + m];
+      const ff keep = up ? w[i + m] : w[i];
+      w[i] = ff_add(keep, shfl_xor_ff(send, h));
+    }
+  }
+  return ff_add(w[0], shfl_xor_ff(w[0], 1));
 }
 
 // ---------------------------------------------------------------------------
@@ -717,12 +750,12 @@ __host__ __device__ __forceinline__ int pupil_scratch_doubles(int n, int sz) {
   const int m1 = n / 2 + 1;
   return 6 * pupil_band_rows(n, sz) * n + 10 * n + 2 * m1 * m1;
 }
-// Warps with a workspace in a per-frame CTA (k_prepare, k_post) and in an
+// Warps with a workspace in a per-frame CTA (k_between) and in an
 // auxiliary CTA for the pupil model: its scratch is ~54 KB per warp at a
 // 30-pixel pupil, ~110 KB at 44 pixels.
 __host__ __device__ __forceinline__ int pupil_ws_warps(int n) { return n <= 30 ? 4 : (n <= 44 ? 2 : 1); }
 
-// Warps of a 1024-thread per-frame CTA (k_prepare, k_post) that carry a
+// Warps of a 1024-thread per-frame CTA (k_between) that carry a
 // workspace: all 32, 8 for the FFT PSF model, whose shape scratch is
 // ~20 KB per warp, and pupil_ws_warps for the pupil model.
 __host__ __device__ __forceinline__ int cta_ws_warps(const ModelCfg& cfg) {
@@ -780,10 +813,37 @@ struct WarpWS {
   float* tab1;  // trial tables (same layout) / pass-1 gradient tables / solve scratch
   double* fw;   // M_FFT / M_PUPIL: the shape evaluation's scratch (fft_scratch_doubles,
                 // pupil_scratch_doubles)
+  float* uh;    // per-pixel terms of the current sums (lm_step_g32): u = t1 rqe psf or a
+  float* ul;    // trial's first-order terms (float-float), the error terms' two factors,
+  float* ps;    // rqe psf (hi, and lo for Z)
+  float* psl;
+  float* dc;
+  float* dr;
+  float* hph;   // H0 psf (float-float)
+  float* hpl;
+  long long* q0f;   // fixed-point words: the start contribution to the fit image and the
+  long long* q0b;   // background sum, and their change by the current trial
+  long long* q1f;
+  long long* q1b;
+  double* anchor;   // the start anchor (x, y) as doubles
   float* par0;  // float-float parameter slots (g32_params) of the step's start record
   float* par1;  // ... and of the current trial
   int ts;       // table stride (ROI size rounded up to 32)
   const unsigned short* roi;   // ROI pixel table (packed rx | ry << 8)
+};
+
+// A team: the warps of one CTA that step one peak together.  Scalars of the
+// step and of the sweep's hand-out, in shared memory.
+constexpr int TEAM_WARPS = 4;
+constexpr int TEAM = 32 * TEAM_WARPS;
+
+struct TeamCtl {
+  double se;      // the step's start error
+  double small;   // tolerance times it (negative: se is not positive)
+  int act;        // the step's next action (warp 0 decides)
+  int r, f;       // the run rank handed out and its frame
+  int li;         // its peak
+  int dil, go, barrier, nb;
 };
 
 template <typename T>
@@ -878,6 +938,53 @@ __device__ inline WarpWS<T> warp_ws(char* base, const ModelCfg& cfg, int nroi) {
   return ws;
 }
 
+// The team workspace of the FP32 Gaussian step: the normal equations, scalars
+// and three records; fixed-point words per pixel (two arrays, four with a
+// camera calibration); the shape tables of the start (4 rows) and of the trial
+// or the Jacobian factors (8 rows, also the scratch of the solver's fallback,
+// 512 bytes); parameter slots; fourteen float arrays per pixel.
+constexpr int G32_FIXED_BYTES = (36 + 16 + 2) * 8 + 3 * (int)sizeof(PeakRec);
+
+__host__ __device__ inline size_t g32_team_bytes(const ModelCfg& cfg) {
+  const size_t n = (size_t)((cfg.nroi + 31) / 32) * 32;
+  const size_t words = (cfg.rqe_one && cfg.scmos_zero) ? 2 : 4;
+  const size_t f = 14 * n + 12 * (size_t)table_stride(cfg.roi) + 2 * 20;
+  return G32_FIXED_BYTES + words * n * sizeof(long long) + ((f * sizeof(float) + 15) & ~(size_t)15);
+}
+
+__device__ inline WarpWS<float> g32_team_ws(char* base, const ModelCfg& cfg) {
+  WarpWS<float> ws{};
+  const size_t n = (size_t)((cfg.nroi + 31) / 32) * 32;
+  const int ts = table_stride(cfg.roi);
+  ws.w = reinterpret_cast<PeakRec*>(base);
+  ws.orig = ws.w + 1;
+  ws.t = ws.w + 2;
+  ws.jh = reinterpret_cast<double*>(base + 3 * sizeof(PeakRec));
+  ws.scratch = ws.jh + 36;
+  ws.anchor = ws.scratch + 16;
+  long long* q = reinterpret_cast<long long*>(base + G32_FIXED_BYTES);
+  ws.q0f = q;
+  ws.q1f = q + n;
+  q += 2 * n;
+  if (!(cfg.rqe_one && cfg.scmos_zero)) {
+    ws.q0b = q;
+    ws.q1b = q + n;
+    q += 2 * n;
+  }
+  float* t = reinterpret_cast<float*>(q);
+  ws.tab1 = t;
+  ws.tab0 = t + 8 * ts;
+  ws.par0 = ws.tab0 + 4 * ts;
+  ws.par1 = ws.par0 + 20;
+  t = ws.par1 + 20;
+  float** arrays[14] = {&ws.t1h, &ws.t1l, &ws.f0g, &ws.T2s, &ws.Rs, &ws.Cs, &ws.uh,
+                        &ws.ul, &ws.ps, &ws.psl, &ws.dc, &ws.dr, &ws.hph, &ws.hpl};
+#pragma unroll
+  for (int i = 0; i < 14; i++) *arrays[i] = t + i * n;
+  ws.ts = ts;
+  return ws;
+}
+
 // ---------------------------------------------------------------------------
 // model pieces (all lanes participate; results in the warp workspace)
 // ---------------------------------------------------------------------------
@@ -952,14 +1059,17 @@ __device__ __forceinline__ ff gpar(const float* par, int slot) { return ff{par[2
 // above e^30 are taken as e^30: a trial with such a factor has a model value
 // of 1e13 or more at that pixel, an error far above any start error, and is
 // rejected whatever the exact value (as the reference rejects it).
+__device__ __forceinline__ ff g32_axis_factor(ff t, ff w) {
+  ff arg = ff_neg(ff_mul(ff_mul(t, t), w));
+  if (arg.h > 30.0f) arg = ff{30.0f, 0.0f};
+  return ff_exp(arg);
+}
+
 __device__ inline void g32_tables_ax(const ModelCfg& cfg, const G32Axes& ax, float* dst, int ts, int lane) {
   for (int i = lane; i < cfg.roi; i += 32) {
     const ff tx = ff_add_f(ax.xo, (float)i), ty = ff_add_f(ax.yo, (float)i);
-    ff argx = ff_neg(ff_mul(ff_mul(tx, tx), ax.wx)), argy = ff_neg(ff_mul(ff_mul(ty, ty), ax.wy));
-    if (argx.h > 30.0f) argx = ff{30.0f, 0.0f};
-    if (argy.h > 30.0f) argy = ff{30.0f, 0.0f};
-    const ff ex = ff_exp(argx);
-    const ff ey = ff_exp(argy);
+    const ff ex = g32_axis_factor(tx, ax.wx);
+    const ff ey = g32_axis_factor(ty, ax.wy);
     dst[i] = ex.h;
     dst[ts + i] = ex.l;
     dst[2 * ts + i] = ey.h;
@@ -983,6 +1093,16 @@ __device__ inline void g32_tables_p(const ModelCfg& cfg, const float* par, float
   g32_tables_ax(cfg, ax, dst, ts, lane);
 }
 
+// One axis' factors alone (hi at dst, lo at dst + ts), one warp.
+static __device__ __noinline__ void g32_table_axis(const ModelCfg& cfg, ff o, ff w, float* dst, int ts, int lane) {
+#pragma unroll 1
+  for (int i = lane; i < cfg.roi; i += 32) {
+    const ff e = g32_axis_factor(ff_add_f(o, (float)i), w);
+    dst[i] = e.h;
+    dst[ts + i] = e.l;
+  }
+}
+
 __device__ __forceinline__ ff g32_psf(const float* tab, int ts, int rx, int ry) {
   return ff_mul(ff{tab[rx], tab[ts + rx]}, ff{tab[2 * ts + ry], tab[3 * ts + ry]});
 }
@@ -991,12 +1111,13 @@ __device__ __forceinline__ ff g32_psf(const float* tab, int ts, int rx, int ry) 
 // f: h * (psf * rqe), bg: bg * rqe + scmos (multi_fit.c:52-54), both
 // float-float.  Every add and subtract of the same record goes through
 // this one function, so they cancel exactly.
+template <bool CALL = false>   // CALL: the conversions out of line
 __device__ __forceinline__ void g32_contrib(const float* tab, int ts, ff H, ff BG, int rx, int ry,
                                             float rq, float sc, Q2& qf, Q2& qb) {
-  const ff ps = ff_mul_f(g32_psf(tab, ts, rx, ry), rq);
-  qf.h = fixed_from_ff(ff_mul(H, ps));
+  const ff vf = ff_mul(H, ff_mul_f(g32_psf(tab, ts, rx, ry), rq)), vb = ff_add_f(ff_mul_f(BG, rq), sc);
+  qf.h = CALL ? fixed_from_ff_call(vf) : fixed_from_ff(vf);
   qf.l = 0;
-  qb.h = fixed_from_ff(ff_add_f(ff_mul_f(BG, rq), sc));
+  qb.h = CALL ? fixed_from_ff_call(vb) : fixed_from_ff(vb);
   qb.l = 0;
 }
 
@@ -2015,16 +2136,17 @@ __device__ __forceinline__ Q2 q_sub(Q2 a, Q2 b) {
 
 // Add (sign +1) or subtract (sign -1) a peak's contribution over its ROI
 // with integer atomics (mFitAddPeak multi_fit.c:28-57, mFitSubtractPeak
-// :1894-1922).  The shape tables of w must be in the workspace.
+// :1894-1922).  The shape tables of w must be in the workspace.  By a warp, or
+// by stride threads of which the caller is thread lane.
 template <typename T>
 __device__ inline void add_peak(const ModelCfg& cfg, const FrameSet<T>& fs, long long fbase,
                                 const PeakRec& w, const SplinePos& s, const WarpWS<T>& ws,
-                                int sign, int lane) {
+                                int sign, int lane, int stride = 32) {
   constexpr int W = AccW<T>::W;
   if constexpr (sizeof(T) == 4) {
     if (!is_spline(cfg.model)) {
       const ff H = ff_from_double(w.p[PH]), BG = ff_from_double(w.p[PBG]);
-      for (int p = lane; p < cfg.nroi; p += 32) {
+      for (int p = lane; p < cfg.nroi; p += stride) {
         int rx, ry;
         roi_rc(fs.roi_xy, p, rx, ry);
         const long long k = pix_index(cfg, w.xi, w.yi, rx, ry);
@@ -2040,7 +2162,7 @@ __device__ inline void add_peak(const ModelCfg& cfg, const FrameSet<T>& fs, long
   if constexpr (sizeof(T) == 4) {
     // FP32 splines
     const ff H = ff_from_double(w.p[PH]), BG = ff_from_double(w.p[PBG]);
-    for (int p = lane; p < cfg.nroi; p += 32) {
+    for (int p = lane; p < cfg.nroi; p += stride) {
       int rx, ry;
       roi_rc(fs.roi_xy, p, rx, ry);
       const long long k = pix_index(cfg, w.xi, w.yi, rx, ry);
@@ -2053,7 +2175,7 @@ __device__ inline void add_peak(const ModelCfg& cfg, const FrameSet<T>& fs, long
     }
     return;
   }
-  for (int p = lane; p < cfg.nroi; p += 32) {
+  for (int p = lane; p < cfg.nroi; p += stride) {
     int rx, ry;
     roi_rc(fs.roi_xy, p, rx, ry);
     const long long k = pix_index(cfg, w.xi, w.yi, rx, ry);

@@ -1,22 +1,24 @@
 // sa_kernels.cuh -- kernels of the GB300 multi-emitter LM engine.
 //
 // One LM sweep (mFitIterateLM, multi_fit.c:1072-1349) over a frame set is
-//   k_prepare   per frame: list RUNNING peaks in index order ("run ranks"),
-//               snapshot them, bin their dilated footprints into a grid
-//               (or, after an escape, roll back and mark barriers)
-//   k_sweep     persistent warps; one warp runs one peak's LM step.  A peak
-//               waits until every lower-index RUNNING peak whose dilated
-//               footprint overlaps its own has finished, which reproduces
-//               the reference's Gauss-Seidel order for every pixel.  A trial
+//   k_sweep     persistent warps; one warp runs one peak's LM step (or
+//   k_sweep_team: a CTA's four warps run one peak's).  A peak waits until
+//               every lower-index RUNNING peak whose dilated footprint
+//               overlaps its own has finished, which reproduces the
+//               reference's Gauss-Seidel order for every pixel.  A trial
 //               step that would leave the footprint "escapes": the peak
 //               restores itself, the frame's later peaks are rolled back and
 //               re-run with the escaped peak as a barrier.
-//   k_post      per frame: recenter (mFitRecenterPeaks :1644-1690), sum the
-//               counters, count RUNNING peaks and decide whether the frame
-//               needs another sweep (dao_fit_c.py:332-356).
+//   k_between   per frame, after a sweep: recenter (mFitRecenterPeaks
+//               :1644-1690), sum the counters, count RUNNING peaks and decide
+//               whether the frame needs another sweep (dao_fit_c.py:332-356);
+//               then list the RUNNING peaks in index order ("run ranks"),
+//               snapshot them and bin their dilated footprints into a grid
+//               (or, after an escape, roll back and mark barriers)
 #pragma once
 
-#include "sa_g32.cuh"
+#include <cstddef>
+#include "sa_g32w.cuh"
 
 namespace sa {
 
@@ -536,13 +538,131 @@ __device__ __forceinline__ bool footprints_overlap(int dx, int dy, int roi, int 
   return ex * ex + ey * ey <= roi * roi;
 }
 
-// G32 >= 0: the FP32 Gaussian step (lm_step_g32) of model G32 (one
+// Waits (one warp, all lanes) until every lower-index RUNNING peak whose
+// dilated footprint overlaps that of run rank r (anchor ax, ay) of frame f
+// has been stepped, in the order the barriers ask for.  barrier: the step is
+// unbounded (index order, or an escaped peak of an earlier attempt).
+// Returns false when a wait timed out (err_flag is set).
+template <typename T>
+__device__ inline bool wait_deps(const ModelCfg& cfg, const FrameSet<T>& fs, FrameCtl* c, int f, int base, int r,
+                                 int ax, int ay, int start, int dil, int nb, int epoch, int lane, bool& barrier) {
+  barrier = c->serial != 0;
+  bool ok = true;
+  // -- dependencies
+  if (c->serial) {
+    if (r - 1 >= start) ok = wait_epoch(fs.done + base + r - 1, epoch, fs.err_flag);
+  } else {
+    // Barriers (escaped peaks of earlier attempts, unbounded steps) are
+    // ascending: the last one <= r decides.  A barrier waits until the
+    // completed prefix reaches it (every lower rank done); a later rank
+    // waits for the last barrier below it, which is done only after
+    // every rank below that barrier.
+    int lo = 0, hi = nb;   // first barrier index with barrier > r
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (c->barrier[mid] <= r) lo = mid + 1;
+      else hi = mid;
+    }
+    const int bprev = lo > 0 ? c->barrier[lo - 1] : -1;
+    if (bprev == r) barrier = true;
+    if (barrier) {
+      ok = wait_prefix(&c->frontier, r, fs.done + base, c->nrun, epoch, fs.err_flag, lane);
+    } else {
+      if (bprev >= start) ok = wait_epoch(fs.done + base + bprev, epoch, fs.err_flag);
+      // lower-index RUNNING neighbours whose dilated footprints overlap:
+      // lane l < 9 reads the range of neighbouring cell l, then the
+      // candidates of all nine cells are checked 32 at a time
+      const int cw = cfg.cell;
+      const int cx = ax / cw, cy = ay / cw;
+      const int* cs = fs.cell_start + (size_t)f * (cfg.gx * cfg.gy + 1);
+      int c0 = 0, cnt = 0;
+      if (lane < 9) {
+        const int yy = cy - 1 + lane / 3, xx = cx - 1 + lane % 3;
+        if (yy >= 0 && yy < cfg.gy && xx >= 0 && xx < cfg.gx) {
+          c0 = cs[yy * cfg.gx + xx];
+          cnt = cs[yy * cfg.gx + xx + 1] - c0;
+        }
+      }
+      int off = cnt;   // inclusive prefix sum over the nine cells
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, off, o);
+        if (lane >= o) off += t;
+      }
+      const int total = __shfl_sync(0xffffffffu, off, 8);
+      off -= cnt;      // exclusive
+      for (int j0 = 0; j0 < total && ok; j0 += 32) {
+        const int j = j0 + lane;
+        // the cell holding candidate j: the last cell whose offset is <= j
+        int idx = -1;
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+          const int ok_ = __shfl_sync(0xffffffffu, off, k);
+          const int ck = __shfl_sync(0xffffffffu, c0, k);
+          if (j < total && j >= ok_) idx = ck + (j - ok_);
+        }
+        int q = -1;
+        if (idx >= 0) {
+          const int2 e = fs.cell_items[base + idx];
+          if (e.x < r && e.x >= start) {
+            const unsigned b0 = (unsigned)e.y;
+            const int bx = b0 & 0xffff, by = b0 >> 16;
+            if (footprints_overlap(bx - ax, by - ay, cfg.roi, dil)) q = e.x;
+          }
+        }
+        // each lane reads its own candidate's done flag (one round trip
+        // for all of them); only the ranks not yet done are waited for,
+        // one at a time by the whole warp.  The __syncwarp orders every
+        // lane's later reads after the lanes' acquire loads.
+        const bool pend = (q >= 0) && (ld_acquire(fs.done + base + q) != epoch);
+        unsigned m = __ballot_sync(0xffffffffu, pend);
+        while (m && ok) {
+          const int src = __ffs(m) - 1;
+          m &= m - 1;
+          const int qq = __shfl_sync(0xffffffffu, q, src);
+          ok = wait_epoch(fs.done + base + qq, epoch, fs.err_flag);
+        }
+        __syncwarp();
+      }
+    }
+  }
+  return ok;
+}
+
+// What the sweep's end needs of a completed step (one warp, after the rank is
+// marked done): the start record for a roll-back, marked with the frame's
+// attempt; the counters added to the frame's; whether the peak goes on and
+// whether it is to be recentered (mFitRecenterPeaks multi_fit.c:1644-1690),
+// so that k_between reads 8 bytes per rank instead of the 128-byte records.
+template <typename T>
+__device__ inline void after_step(const FrameSet<T>& fs, FrameCtl* c, int attempt, int base, int r, int li,
+                                  const PeakRec& start, const PeakRec& end, const int* ctr, int lane) {
+  if (lane < 8) {
+    double2 v = reinterpret_cast<const double2*>(&start)[lane];
+    if (lane == 7) v.x = __hiloint2double(0, attempt);   // pad[0]
+    reinterpret_cast<double2*>(fs.snap + base + li)[lane] = v;
+  }
+  if (lane < NCOUNTERS) {
+    const int v = ctr[lane];
+    if (v) atomicAdd(reinterpret_cast<unsigned long long*>(&c->ctr[lane]), (unsigned long long)v);
+  }
+  // x on lane 0, y on lane 1
+  const double d = lane ? end.p[PY] - end.yi : end.p[PX] - end.xi;
+  const bool out = lane < 2 && (dbl_lt_neg(d, -0.25) || dbl_gt_pos(d, 1.25));
+  const bool moves = __any_sync(0xffffffffu, out);
+  if (lane == 0)
+    fs.after[base + r] = make_int2((int)pack_anchor(end.xi, end.yi),
+                                   end.status == RUNNING ? AFTER_RUNNING | (moves ? AFTER_MOVES : 0) : 0);
+}
+static_assert(offsetof(PeakRec, pad) == 112, "after_step marks PeakRec::pad[0]");
+
+// G32 >= 0: the FP32 Gaussian step (warp32::lm_step_g32) of model G32 (one
 // instantiation per model); G32 < 0: lm_step.
 template <typename T, int G32>
 __global__ void __launch_bounds__(128, 5) k_sweep(ModelCfg cfg, FrameSet<T> fs) {
   extern __shared__ __align__(16) char smem[];
   // the tick's epoch: a done flag equal to it marks a rank done in this
-  // launch (k_post of the previous tick advanced it)
+  // launch (k_between advances it)
   const int epoch = __ldcg(fs.epoch);
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
@@ -577,92 +697,14 @@ __global__ void __launch_bounds__(128, 5) k_sweep(ModelCfg cfg, FrameSet<T> fs) 
     misses = 0;
     const int base = fs.pk_off[f];
     const int start = c->start;
-    const int dil = c->dil;
+    const int dil = c->dil, attempt = c->attempt;
     const unsigned a0 = fs.anchor0[base + r];
     const int ax = a0 & 0xffff, ay = a0 >> 16;
     const int li = fs.run[base + r];
-    if constexpr (G32 >= 0) g32_prologue<G32>(cfg, fs.pk + base + li, ws, lane);
-    bool barrier = c->serial != 0;
-    bool ok = true;
+    if constexpr (G32 >= 0) warp32::g32_prologue<G32>(cfg, fs.pk + base + li, ws, lane);
+    bool barrier;
     const int nb = c->n_barrier;
-    // -- dependencies
-    if (c->serial) {
-      if (r - 1 >= start) ok = wait_epoch(fs.done + base + r - 1, epoch, fs.err_flag);
-    } else {
-      // Barriers (escaped peaks of earlier attempts, unbounded steps) are
-      // ascending: the last one <= r decides.  A barrier waits until the
-      // completed prefix reaches it (every lower rank done); a later rank
-      // waits for the last barrier below it, which is done only after
-      // every rank below that barrier.
-      int lo = 0, hi = nb;   // first barrier index with barrier > r
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (c->barrier[mid] <= r) lo = mid + 1;
-        else hi = mid;
-      }
-      const int bprev = lo > 0 ? c->barrier[lo - 1] : -1;
-      if (bprev == r) barrier = true;
-      if (barrier) {
-        ok = wait_prefix(&c->frontier, r, fs.done + base, c->nrun, epoch, fs.err_flag, lane);
-      } else {
-        if (bprev >= start) ok = wait_epoch(fs.done + base + bprev, epoch, fs.err_flag);
-        // lower-index RUNNING neighbours whose dilated footprints overlap:
-        // lane l < 9 reads the range of neighbouring cell l, then the
-        // candidates of all nine cells are checked 32 at a time
-        const int cw = cfg.cell;
-        const int cx = ax / cw, cy = ay / cw;
-        const int* cs = fs.cell_start + (size_t)f * (cfg.gx * cfg.gy + 1);
-        int c0 = 0, cnt = 0;
-        if (lane < 9) {
-          const int yy = cy - 1 + lane / 3, xx = cx - 1 + lane % 3;
-          if (yy >= 0 && yy < cfg.gy && xx >= 0 && xx < cfg.gx) {
-            c0 = cs[yy * cfg.gx + xx];
-            cnt = cs[yy * cfg.gx + xx + 1] - c0;
-          }
-        }
-        int off = cnt;   // inclusive prefix sum over the nine cells
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, off, o);
-          if (lane >= o) off += t;
-        }
-        const int total = __shfl_sync(0xffffffffu, off, 8);
-        off -= cnt;      // exclusive
-        for (int j0 = 0; j0 < total && ok; j0 += 32) {
-          const int j = j0 + lane;
-          // the cell holding candidate j: the last cell whose offset is <= j
-          int idx = -1;
-#pragma unroll
-          for (int k = 0; k < 9; k++) {
-            const int ok_ = __shfl_sync(0xffffffffu, off, k);
-            const int ck = __shfl_sync(0xffffffffu, c0, k);
-            if (j < total && j >= ok_) idx = ck + (j - ok_);
-          }
-          int q = -1;
-          if (idx >= 0) {
-            const int2 e = fs.cell_items[base + idx];
-            if (e.x < r && e.x >= start) {
-              const unsigned b0 = (unsigned)e.y;
-              const int bx = b0 & 0xffff, by = b0 >> 16;
-              if (footprints_overlap(bx - ax, by - ay, cfg.roi, dil)) q = e.x;
-            }
-          }
-          // each lane reads its own candidate's done flag (one round trip
-          // for all of them); only the ranks not yet done are waited for,
-          // one at a time by the whole warp.  The __syncwarp orders every
-          // lane's later reads after the lanes' acquire loads.
-          const bool pend = (q >= 0) && (ld_acquire(fs.done + base + q) != epoch);
-          unsigned m = __ballot_sync(0xffffffffu, pend);
-          while (m && ok) {
-            const int src = __ffs(m) - 1;
-            m &= m - 1;
-            const int qq = __shfl_sync(0xffffffffu, q, src);
-            ok = wait_epoch(fs.done + base + qq, epoch, fs.err_flag);
-          }
-          __syncwarp();
-        }
-      }
-    }
+    const bool ok = wait_deps(cfg, fs, c, f, base, r, ax, ay, start, dil, nb, epoch, lane, barrier);
     if (!ok) return;   // a wait timed out: err_flag is set, the host reports it
     // A lower rank of this attempt escaped: every rank above it re-runs in
     // the next attempt, so this one is skipped now (record and image stay
@@ -679,8 +721,8 @@ __global__ void __launch_bounds__(128, 5) k_sweep(ModelCfg cfg, FrameSet<T> fs) 
     // -- the step
     bool esc;
     if constexpr (G32 >= 0)
-      esc = lm_step_g32<G32>(cfg, fs, (long long)f * fs.npix, fs.pk + base + li, barrier, dil, ws,
-                             fs.stepctr + (size_t)(base + li) * NCOUNTERS, lane);
+      esc = warp32::lm_step_g32<G32>(cfg, fs, (long long)f * fs.npix, fs.pk + base + li, barrier, dil, ws,
+                                     fs.stepctr + (size_t)(base + li) * NCOUNTERS, lane);
     else
       esc = lm_step(cfg, fs, (long long)f * fs.npix, fs.pk + base + li, barrier, dil, ws,
                     fs.stepctr + (size_t)(base + li) * NCOUNTERS, lane);
@@ -693,110 +735,286 @@ __global__ void __launch_bounds__(128, 5) k_sweep(ModelCfg cfg, FrameSet<T> fs) 
     __syncwarp();
     if (lane == 0) st_release(fs.done + base + r, epoch);
     if (nb > 0) advance_prefix(&c->frontier, fs.done + base, c->nrun, epoch, lane);
+    if (!esc) {
+      const int* ctr = fs.stepctr + (size_t)(base + li) * NCOUNTERS;
+      if constexpr (G32 >= 0) ctr = reinterpret_cast<const int*>(ws.scratch);
+      after_step(fs, c, attempt, base, r, li, *ws.orig, *ws.w, ctr, lane);
+    }
+    __syncwarp();
   }
 }
 
 // ---------------------------------------------------------------------------
-// k_prepare: one CTA (1024 threads) per frame
+// k_sweep_team: the same sweep with a team (one CTA) per peak
 // ---------------------------------------------------------------------------
 
+// Hand out the next run rank (one warp): 32 frames are looked at per round
+// trip, from frame f on (a warp that looked at one frame at a time spent
+// ~0.7 us on each exhausted frame, 64 of them at the end of every sweep of
+// the benchmark batch).  Returns the rank and sets f, or -1 when every frame
+// is exhausted.
 template <typename T>
-__global__ void __launch_bounds__(1024) k_prepare(ModelCfg cfg, FrameSet<T> fs) {
+__device__ inline int grab_rank(const FrameSet<T>& fs, int& f, int lane) {
+  for (int k0 = 0; k0 < fs.F; k0 += 32) {
+    int q = f + k0 + lane;
+    if (q >= fs.F) q -= fs.F;
+    int nrun = 0;
+    if (k0 + lane < fs.F) {
+      FrameCtl* c = fs.ctl + q;
+      // plain reads first: exhausted frames cost no atomic
+      const int ph = *((volatile int*)&c->phase), gr = *((volatile int*)&c->grab), nr = *((volatile int*)&c->nrun);
+      if (ph == PH_IN_SWEEP && gr < nr) nrun = nr;
+    }
+    unsigned m = __ballot_sync(0xffffffffu, nrun > 0);
+    while (m) {
+      const int src = __ffs(m) - 1;
+      m &= m - 1;
+      const int qf = __shfl_sync(0xffffffffu, q, src), qn = __shfl_sync(0xffffffffu, nrun, src);
+      int r = 0;
+      if (lane == 0) r = atomicAdd(&fs.ctl[qf].grab, 1);
+      r = __shfl_sync(0xffffffffu, r, 0);
+      if (r < qn) {
+        f = qf;
+        return r;
+      }
+    }
+  }
+  return -1;
+}
+
+template <int M>
+__global__ void __launch_bounds__(TEAM, 8) k_sweep_team(ModelCfg cfg, FrameSet<float> fs) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ TeamCtl tc;
+  const int epoch = __ldcg(fs.epoch);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  WarpWS<float> ws = g32_team_ws(smem, cfg);
+  {
+    unsigned short* roi = reinterpret_cast<unsigned short*>(smem + g32_team_bytes(cfg));
+    for (int i = tid; i < cfg.nroi; i += TEAM) roi[i] = fs.roi_xy[i];
+    ws.roi = roi;
+  }
+  int fcur = blockIdx.x % fs.F;   // warp 0's
+  for (;;) {
+    if (wid == 0) {
+      const int r = grab_rank(fs, fcur, lane);
+      if (lane == 0) {
+        tc.r = r;
+        if (r >= 0) {
+          tc.f = fcur;
+          tc.li = fs.run[fs.pk_off[fcur] + r];
+        }
+      }
+    }
+    __syncthreads();
+    const int r = tc.r;
+    if (r < 0) return;
+    const int f = tc.f, li = tc.li;
+    const int base = fs.pk_off[f];
+    FrameCtl* c = fs.ctl + f;
+    // warp 3 waits for the step's predecessors while the others compute what
+    // the step needs of its own record
+    if (wid < 3) {
+      g32_prologue<M, 3>(cfg, fs, fs.pk + base + li, ws, tid);
+    } else {
+      const int start = c->start, dil = c->dil, nb = c->n_barrier;
+      const unsigned a0 = fs.anchor0[base + r];
+      bool barrier;
+      const bool ok = wait_deps(cfg, fs, c, f, base, r, a0 & 0xffff, a0 >> 16, start, dil, nb, epoch, lane, barrier);
+      if (lane == 0) {
+        // 0: a wait timed out (err_flag is set, the host reports it); 2: a
+        // lower rank of this attempt escaped, so every rank above it re-runs
+        // in the next attempt and this one is skipped now (record and image
+        // stay as they are, nothing to roll back); 1: step
+        tc.go = !ok ? 0 : (*((volatile int*)&c->escaped_min) < r ? 2 : 1);
+        tc.barrier = barrier;
+        tc.dil = dil;
+        tc.nb = nb;
+      }
+    }
+    // No fence before the step: warp 3's acquire loads of the dependencies'
+    // done flags, and this barrier, order the step's reads after the
+    // predecessors' writes.
+    __syncthreads();
+    const int go = tc.go;
+    if (go == 0) return;
+    bool esc = false;
+    if (go == 1)
+      esc = lm_step_g32<M>(cfg, fs, (long long)f * fs.npix, fs.pk + base + li, tc.barrier != 0, tc.dil, ws, tc,
+                           fs.stepctr + (size_t)(base + li) * NCOUNTERS, tid);
+    __syncthreads();
+    if (wid == 0) {
+      if (lane == 0) {
+        if (esc) {
+          atomicMin(&c->escaped_min, r);
+          const int slot = atomicAdd(&c->n_escaped, 1);
+          if (slot < MAX_ESCAPES) c->escaped[slot] = r;
+        }
+        // the barrier above put the team's writes before this fence
+        __threadfence();
+        st_release(fs.done + base + r, epoch);
+      }
+      __syncwarp();
+      if (tc.nb > 0) advance_prefix(&c->frontier, fs.done + base, c->nrun, epoch, lane);
+      if (go == 1 && !esc)
+        after_step(fs, c, c->attempt, base, r, li, *ws.orig, tc.act == ACT_BREAK_ADDED ? *ws.t : *ws.w,
+                   reinterpret_cast<const int*>(ws.scratch), lane);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// k_between: one CTA (1024 threads) per frame
+// ---------------------------------------------------------------------------
+
+// A per-frame CTA's workspace w (of cta_ws_warps).
+template <typename T>
+__device__ __forceinline__ WarpWS<T> cta_ws(const ModelCfg& cfg, char* smem, int w) {
+  return warp_ws<T>(smem + (size_t)w * warp_ws_bytes<T>(cfg, 0), cfg, 0);
+}
+
+// Recentre one peak that left its window (mFitRecenterPeaks multi_fit.c:
+// 1644-1690; one warp).  Returns 0 (RUNNING), else base_check's code (the peak
+// is then ERROR).  Out of line, as what follows: its registers would spill
+// the pass's.
+template <typename T>
+__device__ __noinline__ int recenter_peak_warp(const ModelCfg& cfg, const FrameSet<T>& fs, long long fbase,
+                                               PeakRec* recp, char* smem, int wid, int lane) {
+  PeakRec rec;
+  load_rec(recp, rec);
+  WarpWS<T> ws = cta_ws<T>(cfg, smem, wid);
+  SplinePos s = shape_tables(cfg, rec, ws, lane);
+  add_peak(cfg, fs, fbase, rec, s, ws, -1, lane);
+  __syncwarp();
+  rec.added -= 1;
+  rec.xi = (int)floor(rec.p[PX]);
+  rec.yi = (int)floor(rec.p[PY]);
+  const int chk = base_check(cfg, rec);
+  if (chk) {
+    rec.status = ERROR;
+  } else {
+    s = shape_tables(cfg, rec, ws, lane);
+    add_peak(cfg, fs, fbase, rec, s, ws, +1, lane);
+    rec.added += 1;
+  }
+  __syncwarp();
+  if (lane == 0) *recp = rec;
+  return chk;
+}
+
+// The same by the whole CTA, its pixels a thread each.
+template <typename T>
+__device__ __noinline__ int recenter_peak(const ModelCfg& cfg, const FrameSet<T>& fs, long long fbase, PeakRec* recp,
+                                          char* smem, PeakRec* s_rec) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid < 8) reinterpret_cast<double2*>(s_rec)[tid] = __ldcg(reinterpret_cast<const double2*>(recp) + tid);
+  __syncthreads();
+  PeakRec rec = s_rec[0], to = s_rec[0];
+  to.added = rec.added - 1;
+  to.xi = (int)floor(rec.p[PX]);
+  to.yi = (int)floor(rec.p[PY]);
+  const int chk = base_check(cfg, to);
+  if (chk) to.status = ERROR;
+  else to.added += 1;
+  // the tables of the two anchors in workspaces 0 and 1, or one after the other
+  const bool two = cta_ws_warps(cfg) > 1;
+  const WarpWS<T> w0 = cta_ws<T>(cfg, smem, 0), w1 = cta_ws<T>(cfg, smem, two ? 1 : 0);
+  if (wid == 0) {
+    WarpWS<T> w = w0;
+    shape_tables(cfg, rec, w, lane);
+  } else if (wid == 1 && two && !chk) {
+    WarpWS<T> w = w1;
+    shape_tables(cfg, to, w, lane);
+  }
+  __syncthreads();
+  SplinePos s{};
+  if (is_spline(cfg.model)) s = spline_pos(rec.p, rec.xi, rec.yi, rec.zi);
+  add_peak(cfg, fs, fbase, rec, s, w0, -1, tid, blockDim.x);
+  if (!chk) {
+    if (!two) {
+      __syncthreads();
+      if (wid == 0) {
+        WarpWS<T> w = w1;
+        shape_tables(cfg, to, w, lane);
+      }
+      __syncthreads();
+    }
+    if (is_spline(cfg.model)) s = spline_pos(to.p, to.xi, to.yi, to.zi);
+    add_peak(cfg, fs, fbase, to, s, w1, +1, tid, blockDim.x);
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) *recp = to;
+  return chk;
+}
+
+// Take a peak stepped in this attempt back to its record at the sweep's start
+// (one warp): remove the current contribution, restore the snapshot, take
+// its counters back.
+template <typename T>
+__device__ __noinline__ void roll_back_peak(const ModelCfg& cfg, const FrameSet<T>& fs, FrameCtl* c, long long fbase,
+                                            int slot, char* smem, int wid, int lane) {
+  PeakRec cur, sn;
+  load_rec(fs.snap + slot, sn);
+  // ranks skipped after the escape, or escaped themselves, are untouched
+  if (sn.pad[0] != c->attempt) return;
+  sn.pad[0] = 0;
+  load_rec(fs.pk + slot, cur);
+  WarpWS<T> ws = cta_ws<T>(cfg, smem, wid);
+  if (cur.added > 0) {
+    SplinePos s = shape_tables(cfg, cur, ws, lane);
+    add_peak(cfg, fs, fbase, cur, s, ws, -1, lane);
+  }
+  __syncwarp();
+  if (sn.added > 0) {
+    SplinePos s = shape_tables(cfg, sn, ws, lane);
+    add_peak(cfg, fs, fbase, sn, s, ws, +1, lane);
+  }
+  __syncwarp();
+  if (lane == 0) fs.pk[slot] = sn;
+  if (lane < NCOUNTERS) {
+    const long long v = fs.stepctr[(size_t)slot * NCOUNTERS + lane];
+    if (v) atomicAdd(reinterpret_cast<unsigned long long*>(&c->ctr[lane]), (unsigned long long)(-v));
+  }
+}
+
+// What lies between two sweeps of a frame: the end of the one before (frames
+// IN_SWEEP) and the set-up of the next, in one pass over the run ranks.
+// start_only: only the frames whose fit starts (SWEEP_PENDING).  poll: where
+// the frames' states and the error flag are left for the host (or null).
+//
+// Bound by its chain of round trips and by fetching code that runs once:
+// one CTA per frame, alone on the GPU between two sweeps of a lone frame.
+// Reading what the steps left (FrameSet::after) instead of their records and
+// counters, and leaving the start records to the steps, took it from 70 us
+// to 11 at 2,000 ranks and from 16 to 7 at 200 (no peak to recenter).
+template <typename T>
+__global__ void __launch_bounds__(1024)
+    k_between(const __grid_constant__ ModelCfg cfg, const __grid_constant__ FrameSet<T> fs, int start_only,
+              FramePoll* poll, unsigned* poll_err) {
   extern __shared__ __align__(16) char smem[];
   __shared__ int sc32[33];
-  __shared__ int s_total;
+  __shared__ int s_nmove;
+  __shared__ int s_move[1024];
+  __shared__ PeakRec s_rec;
   const int f = blockIdx.x;
   FrameCtl* c = fs.ctl + f;
-  const int phase = c->phase;
-  const int base = fs.pk_off[f];
   const int tid = threadIdx.x;
-  if (phase == PH_SWEEP_PENDING) {
-    // Within a fit a peak only leaves RUNNING, so after the first sweep the
-    // candidates are the previous sweep's run list (compacted in place:
-    // every kept entry moves to a lower or equal position, and a chunk is
-    // read before any of it is written).
-    const bool from_run = c->sweeps > 0;
-    const int n = from_run ? c->nrun : fs.nfit[f];
-    int nrun = 0;
-    for (int c0 = 0; c0 < n; c0 += 1024) {
-      const int k = c0 + tid;
-      const int i = (k < n) ? (from_run ? fs.run[base + k] : k) : -1;
-      __syncthreads();
-      int flag = 0;
-      if (i >= 0 && fs.pk[base + i].status == RUNNING) {
-        // A RUNNING peak always has an in-image ROI, except one re-marked
-        // RUNNING by the caller after a failed placement; it cannot be
-        // fitted (its ROI is outside the image) and is set to ERROR.
-        const PeakRec& q = fs.pk[base + i];
-        if (q.xi < 0 || q.yi < 0 || q.xi >= cfg.nx - cfg.roi || q.yi >= cfg.ny - cfg.roi)
-          fs.pk[base + i].status = ERROR;
-        else
-          flag = 1;
-      }
-      int tot;
-      const int pos = block_excl_scan(flag, sc32, tot);
-      if (flag) {
-        const PeakRec& rec = fs.pk[base + i];
-        fs.run[base + nrun + pos] = i;
-        fs.snap[base + i] = rec;
-        fs.anchor0[base + nrun + pos] = pack_anchor(rec.xi, rec.yi);
-      }
-      nrun += tot;
-    }
-    // grid of dilated-footprint anchors (counting sort by cell)
-    const int ncell = cfg.gx * cfg.gy;
-    int* cntc = reinterpret_cast<int*>(smem);
-    for (int i = tid; i < ncell; i += 1024) cntc[i] = 0;
-    __syncthreads();
-    for (int r = tid; r < nrun; r += 1024) {
-      const unsigned a = fs.anchor0[base + r];
-      const int cell = ((a >> 16) / cfg.cell) * cfg.gx + (a & 0xffff) / cfg.cell;
-      atomicAdd(&cntc[cell], 1);
-    }
-    __syncthreads();
-    int* cs = fs.cell_start + (size_t)f * (ncell + 1);
-    // exclusive scan of ncell counts: per-thread contiguous chunk
-    const int per = (ncell + 1023) / 1024;
-    const int lo = tid * per, hi = min(lo + per, ncell);
-    int local = 0;
-    for (int i = lo; i < hi; i++) local += cntc[i];
-    int tot;
-    int off = block_excl_scan(local, sc32, tot);
-    for (int i = lo; i < hi; i++) {
-      const int v = cntc[i];
-      cs[i] = off;
-      cntc[i] = off;   // becomes the fill cursor
-      off += v;
-    }
-    if (tid == 0) cs[ncell] = tot;
-    __syncthreads();
-    for (int r = tid; r < nrun; r += 1024) {
-      const unsigned a = fs.anchor0[base + r];
-      const int cell = ((a >> 16) / cfg.cell) * cfg.gx + (a & 0xffff) / cfg.cell;
-      const int slot = atomicAdd(&cntc[cell], 1);
-      fs.cell_items[base + slot] = make_int2(r, (int)a);
-    }
-    if (tid == 0) {
-      c->nrun = nrun;
-      c->start = 0;
-      c->grab = 0;
-      c->frontier = 0;
-      c->escaped_min = INT_MAX;
-      c->n_escaped = 0;
-      c->n_barrier = 0;
-      c->serial = cfg.force_serial;
-      // the late dilation from sweep dil_switch on, unless the previous
-      // sweep of this frame re-ran more than once (anchors still moving
-      // in many places: a dense frame then spends more on re-runs than
-      // the wider footprints cost)
-      c->dil = (c->sweeps >= cfg.dil_switch && c->attempts <= 2) ? cfg.dil_late : cfg.dil;
-      c->attempts = 1;
-      c->phase = nrun > 0 ? PH_IN_SWEEP : PH_IN_SWEEP;
-    }
-  } else if (phase == PH_RERUN_PENDING) {
-    const int b = c->escaped_min;
-    const int nrun = c->nrun;
-    // barriers: merge the escaped run ranks
+  // the next sweep's epoch (every sweep of this tick has finished)
+  if (f == 0 && tid == 0 && !start_only) *fs.epoch += 1;
+  const int phase = c->phase, sweeps = c->sweeps, n_last = c->nrun, max_sweeps = c->max_sweeps;
+  const int escaped_min = c->escaped_min, attempts = c->attempts;
+  const int base = fs.pk_off[f];
+  const bool first = phase == PH_SWEEP_PENDING;
+  if (poll && f == 0 && tid == 0) *poll_err = __ldcg(fs.err_flag);
+  if (!first && (start_only || phase != PH_IN_SWEEP)) {
+    if (poll && tid == 0) poll[f] = FramePoll{phase, sweeps, c->unconverged, n_last};
+    return;
+  }
+  const long long fbase = (long long)f * fs.npix;
+  if (!first && escaped_min != INT_MAX) {
+    // -- the attempt had escapes: again from the lowest escaped rank
+    const int b = escaped_min;
     if (tid == 0) {
       // merge the escaped run ranks into the ascending barrier list
       const int ne = min(c->n_escaped, MAX_ESCAPES);
@@ -814,38 +1032,11 @@ __global__ void __launch_bounds__(1024) k_prepare(ModelCfg cfg, FrameSet<T> fs) 
         c->n_barrier++;
       }
       if (c->n_escaped > MAX_ESCAPES) c->serial = 1;
-      s_total = 0;
     }
-    __syncthreads();
-    // roll back run ranks > b: remove the current contribution, restore the snapshot
-    const int lane = tid & 31, wid = tid >> 5;
-    const int nws = cta_ws_warps(cfg);
-    WarpWS<T> ws = warp_ws<T>(smem + (size_t)(wid < nws ? wid : 0) * warp_ws_bytes<T>(cfg, 0), cfg, 0);
-    const long long fbase = (long long)f * fs.npix;
-    for (int r = b + 1 + wid; wid < nws && r < nrun; r += nws) {
-      const int li = fs.run[base + r];
-      PeakRec cur, sn;
-      load_rec(fs.pk + base + li, cur);
-      load_rec(fs.snap + base + li, sn);
-      // ranks skipped after the escape (or escaped themselves) are untouched
-      bool same = true;
-      const long long* wa = reinterpret_cast<const long long*>(&cur);
-      const long long* wb = reinterpret_cast<const long long*>(&sn);
-#pragma unroll
-      for (int q = 0; q < (int)(sizeof(PeakRec) / 8); q++) same = same && (wa[q] == wb[q]);
-      if (same) continue;
-      if (cur.added > 0) {
-        SplinePos s = shape_tables(cfg, cur, ws, lane);
-        add_peak(cfg, fs, fbase, cur, s, ws, -1, lane);
-      }
-      __syncwarp();
-      if (sn.added > 0) {
-        SplinePos s = shape_tables(cfg, sn, ws, lane);
-        add_peak(cfg, fs, fbase, sn, s, ws, +1, lane);
-      }
-      __syncwarp();
-      if (lane == 0) fs.pk[base + li] = sn;
-    }
+    // roll back run ranks > b
+    const int nws = cta_ws_warps(cfg), wid = tid >> 5;
+    for (int r = b + 1 + wid; wid < nws && r < n_last; r += nws)
+      roll_back_peak(cfg, fs, c, fbase, base + fs.run[base + r], smem, wid, tid & 31);
     __threadfence();
     __syncthreads();
     if (tid == 0) {
@@ -854,119 +1045,144 @@ __global__ void __launch_bounds__(1024) k_prepare(ModelCfg cfg, FrameSet<T> fs) 
       c->frontier = b;
       c->escaped_min = INT_MAX;
       c->n_escaped = 0;
-      c->attempts += 1;
+      c->attempts = attempts + 1;
+      c->attempt += 1;
       c->reruns_total += 1;
       c->barriers_total = c->barriers_total + c->n_barrier;
-      c->phase = PH_IN_SWEEP;
+      if (poll) poll[f] = FramePoll{phase, sweeps, c->unconverged, n_last};
     }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// k_post: one CTA (1024 threads) per frame
-// ---------------------------------------------------------------------------
-
-template <typename T>
-__global__ void __launch_bounds__(1024) k_post(ModelCfg cfg, FrameSet<T> fs) {
-  extern __shared__ __align__(16) char smem[];
-  __shared__ long long s_ctr[NCOUNTERS];
-  __shared__ int s_unconv;
-  __shared__ int s_nmove;
-  __shared__ int s_move[1024];
-  const int f = blockIdx.x;
-  FrameCtl* c = fs.ctl + f;
-  // the next tick's epoch (every k_sweep of this tick has finished)
-  if (f == 0 && threadIdx.x == 0) *fs.epoch += 1;
-  if (c->phase != PH_IN_SWEEP) return;
-  const int tid = threadIdx.x;
-  if (c->escaped_min != INT_MAX) {
-    __syncthreads();
-    if (tid == 0) c->phase = PH_RERUN_PENDING;
     return;
   }
-  if (tid < NCOUNTERS) s_ctr[tid] = 0;
-  if (tid == 0) s_unconv = 0;
-  __syncthreads();
-  const int base = fs.pk_off[f];
-  const int nrun = c->nrun;
-  const int lane = tid & 31, wid = tid >> 5;
-  const int nws = cta_ws_warps(cfg);
-  WarpWS<T> ws = warp_ws<T>(smem + (size_t)(wid < nws ? wid : 0) * warp_ws_bytes<T>(cfg, 0), cfg, 0);
-  const long long fbase = (long long)f * fs.npix;
-  // recenter (mFitRecenterPeaks multi_fit.c:1644-1690); order-free with
-  // fixed-point accumulation.  The run ranks are scanned a thread each; the
-  // peaks that move their ROI are listed and then re-added a warp each.
-  int lost = 0, margin = 0, negh = 0, unconv = 0;
-  for (int c0 = 0; c0 < nrun; c0 += 1024) {
-    if (tid == 0) s_nmove = 0;
+
+  // -- one pass over the candidates.  Within a fit a peak only leaves RUNNING,
+  // so after the first sweep the candidates are the previous sweep's run list
+  // (compacted in place: every kept entry moves to a lower or equal position,
+  // and a chunk is read before any of it is written).  Recentering is
+  // order-free with fixed-point accumulation.
+  const bool all = first && sweeps == 0;
+  const int n = all ? fs.nfit[f] : n_last;
+  if (tid == 0) s_nmove = 0;
+  int nrun = 0;
+  for (int c0 = 0; c0 < n; c0 += 1024) {
+    const int k = c0 + tid;
+    int i = -1, anchor = 0;
+    bool flag = false;
     __syncthreads();
-    const int rr = c0 + tid;
-    if (rr < nrun) {
-      const PeakRec* q = fs.pk + base + fs.run[base + rr];
-      if (__ldcg(&q->status) == RUNNING) {
-        const double dx = __ldcg(&q->p[PX]) - __ldcg(&q->xi), dy = __ldcg(&q->p[PY]) - __ldcg(&q->yi);
-        if ((dx < -0.25) || (dx > 1.25) || (dy < -0.25) || (dy > 1.25)) s_move[atomicAdd(&s_nmove, 1)] = rr;
-        else unconv++;
-      }
-    }
-    __syncthreads();
-    const int nmove = s_nmove;
-    for (int m = wid; wid < nws && m < nmove; m += nws) {
-      const int li = fs.run[base + s_move[m]];
-      PeakRec rec;
-      load_rec(fs.pk + base + li, rec);
-      SplinePos s = shape_tables(cfg, rec, ws, lane);
-      add_peak(cfg, fs, fbase, rec, s, ws, -1, lane);
-      __syncwarp();
-      rec.added -= 1;
-      rec.xi = (int)floor(rec.p[PX]);
-      rec.yi = (int)floor(rec.p[PY]);
-      const int chk = base_check(cfg, rec);
-      if (chk) {
-        if (lane == 0) {
-          lost++;
-          if (chk == 1) margin++;
-          else negh++;
+    if (k < n) {
+      i = all ? k : fs.run[base + k];
+      if (first) {
+        const PeakRec& q = fs.pk[base + i];
+        flag = q.status == RUNNING;
+        anchor = (int)pack_anchor(q.xi, q.yi);
+        // A RUNNING peak always has an in-image ROI, except one re-marked
+        // RUNNING by the caller after a failed placement; it cannot be
+        // fitted (its ROI is outside the image) and is set to ERROR.
+        if (flag && (q.xi < 0 || q.yi < 0 || q.xi >= cfg.nx - cfg.roi || q.yi >= cfg.ny - cfg.roi)) {
+          fs.pk[base + i].status = ERROR;
+          flag = false;
         }
-        rec.status = ERROR;
       } else {
-        SplinePos s2 = shape_tables(cfg, rec, ws, lane);
-        add_peak(cfg, fs, fbase, rec, s2, ws, +1, lane);
-        rec.added += 1;
-      }
-      __syncwarp();
-      if (lane == 0) {
-        fs.pk[base + li] = rec;
-        if (rec.status == RUNNING) unconv++;
+        const int2 a = fs.after[base + k];
+        anchor = a.x;
+        flag = (a.y & AFTER_RUNNING) != 0;
+        if (a.y & AFTER_MOVES) {
+          s_move[atomicAdd(&s_nmove, 1)] = i;
+          anchor = -1;   // not a packed anchor: known once it has moved
+        }
       }
     }
     __syncthreads();
+    if (s_nmove > 0) {
+      // One or two peaks by the whole CTA, more a peak per warp: 14 us a
+      // peak against ~40 us a round of up to 32 (the first sweeps of a frame
+      // of 3,355 peaks move about a hundred each).
+      const int nmove = s_nmove, nws = cta_ws_warps(cfg), wid = tid >> 5;
+      const bool cta = nmove <= 2;
+      for (int m = cta ? 0 : wid; (cta || wid < nws) && m < nmove; m += cta ? 1 : nws) {
+        PeakRec* q = fs.pk + base + s_move[m];
+        const int chk = cta ? recenter_peak(cfg, fs, fbase, q, smem, &s_rec)
+                            : recenter_peak_warp(cfg, fs, fbase, q, smem, wid, tid & 31);
+        if (chk && (cta ? tid == 0 : (tid & 31) == 0)) {
+          atomicAdd(reinterpret_cast<unsigned long long*>(&c->ctr[C_LOST]), 1ull);
+          atomicAdd(reinterpret_cast<unsigned long long*>(&c->ctr[chk == 1 ? C_MARGIN : C_NEGH]), 1ull);
+        }
+      }
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) s_nmove = 0;
+      if (flag && anchor == -1) {
+        const PeakRec* q = fs.pk + base + i;
+        flag = __ldcg(&q->status) == RUNNING;
+        anchor = (int)pack_anchor(__ldcg(&q->xi), __ldcg(&q->yi));
+      }
+    }
+    int tot;
+    const int pos = block_excl_scan(flag, sc32, tot);
+    if (flag) {
+      fs.run[base + nrun + pos] = i;
+      fs.anchor0[base + nrun + pos] = (unsigned)anchor;
+    }
+    nrun += tot;
   }
-  // counters of this sweep's steps
-  long long loc[NCOUNTERS];
-  for (int i = 0; i < NCOUNTERS; i++) loc[i] = 0;
-  for (int r = tid; r < nrun; r += 1024) {
-    const int li = fs.run[base + r];
-    const int* sc = fs.stepctr + (size_t)(base + li) * NCOUNTERS;
-    for (int i = 0; i < NCOUNTERS; i++) loc[i] += sc[i];
-  }
-  loc[C_LOST] += lost;
-  loc[C_MARGIN] += margin;
-  loc[C_NEGH] += negh;
-  for (int i = 0; i < NCOUNTERS; i++) {
-    long long v = loc[i];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0 && v) atomicAdd(reinterpret_cast<unsigned long long*>(&s_ctr[i]), (unsigned long long)v);
-  }
-  for (int o = 16; o > 0; o >>= 1) unconv += __shfl_xor_sync(0xffffffffu, unconv, o);
-  if (lane == 0 && unconv) atomicAdd(&s_unconv, unconv);
-  __threadfence();
-  __syncthreads();
+  const int done_sweeps = sweeps + (first ? 0 : 1);
+  const bool done = !first && (nrun == 0 || done_sweeps >= max_sweeps);
   if (tid == 0) {
-    for (int i = 0; i < NCOUNTERS; i++) c->ctr[i] += s_ctr[i];
-    c->unconverged = s_unconv;
-    c->sweeps += 1;
-    c->phase = (s_unconv == 0 || c->sweeps >= c->max_sweeps) ? PH_DONE : PH_SWEEP_PENDING;
+    c->sweeps = done_sweeps;
+    if (!first) c->unconverged = nrun;
+    c->nrun = nrun;
+    c->phase = done ? PH_DONE : PH_IN_SWEEP;
+    if (poll) poll[f] = FramePoll{done ? PH_DONE : PH_IN_SWEEP, done_sweeps, first ? c->unconverged : nrun, nrun};
+    if (!done) {
+      c->start = 0;
+      c->grab = 0;
+      c->frontier = 0;
+      c->escaped_min = INT_MAX;
+      c->n_escaped = 0;
+      c->n_barrier = 0;
+      c->serial = cfg.force_serial;
+      // the late dilation from sweep dil_switch on, unless the previous
+      // sweep of this frame re-ran more than once (anchors still moving
+      // in many places: a dense frame then spends more on re-runs than
+      // the wider footprints cost)
+      c->dil = (done_sweeps >= cfg.dil_switch && attempts <= 2) ? cfg.dil_late : cfg.dil;
+      c->attempts = 1;
+      c->attempt += 1;
+    }
+  }
+  if (done) return;
+
+  // -- grid of dilated-footprint anchors (counting sort by cell)
+  const int ncell = cfg.gx * cfg.gy;
+  int* cntc = reinterpret_cast<int*>(smem);
+  for (int i = tid; i < ncell; i += 1024) cntc[i] = 0;
+  __syncthreads();
+  for (int r = tid; r < nrun; r += 1024) {
+    const unsigned a = fs.anchor0[base + r];
+    const int cell = ((a >> 16) / cfg.cell) * cfg.gx + (a & 0xffff) / cfg.cell;
+    atomicAdd(&cntc[cell], 1);
+  }
+  __syncthreads();
+  int* cs = fs.cell_start + (size_t)f * (ncell + 1);
+  // exclusive scan of ncell counts: per-thread contiguous chunk
+  const int per = (ncell + 1023) / 1024;
+  const int lo = min(tid * per, ncell), hi = min(lo + per, ncell);
+  int local = 0;
+  for (int i = lo; i < hi; i++) local += cntc[i];
+  int tot;
+  int off = block_excl_scan(local, sc32, tot);
+  for (int i = lo; i < hi; i++) {
+    const int v = cntc[i];
+    cs[i] = off;
+    cntc[i] = off;   // becomes the fill cursor
+    off += v;
+  }
+  if (tid == 0) cs[ncell] = tot;
+  __syncthreads();
+  for (int r = tid; r < nrun; r += 1024) {
+    const unsigned a = fs.anchor0[base + r];
+    const int cell = ((a >> 16) / cfg.cell) * cfg.gx + (a & 0xffff) / cfg.cell;
+    const int slot = atomicAdd(&cntc[cell], 1);
+    fs.cell_items[base + slot] = make_int2(r, (int)a);
   }
 }
 
@@ -974,9 +1190,93 @@ __global__ void __launch_bounds__(1024) k_post(ModelCfg cfg, FrameSet<T> fs) {
 // k_tail: the remaining sweeps of frames with few RUNNING peaks, one launch
 // ---------------------------------------------------------------------------
 
+// Whether a frame is k_tail's: set up for a sweep (k_between, its first
+// attempt) of at most tail_peaks peaks, after at least one.
+__device__ __forceinline__ bool tail_ready(const FrameCtl* c, int tail_peaks) {
+  return c->phase == PH_IN_SWEEP && c->sweeps > 0 && c->start == 0 && c->n_barrier == 0 && c->nrun <= tail_peaks;
+}
+
+// The run list of a tail sweep (one warp): the previous run list's RUNNING
+// peaks, in order (k_between).  Returns their number.
+template <typename T>
+__device__ inline int tail_run_list(const ModelCfg& cfg, const FrameSet<T>& fs, int base, int nrun, int lane) {
+  int m = 0;
+  for (int k0 = 0; k0 < nrun; k0 += 32) {
+    const int k = k0 + lane;
+    const int i = (k < nrun) ? fs.run[base + k] : -1;
+    bool flag = false;
+    if (i >= 0 && fs.pk[base + i].status == RUNNING) {
+      const PeakRec& q = fs.pk[base + i];
+      if (q.xi < 0 || q.yi < 0 || q.xi >= cfg.nx - cfg.roi || q.yi >= cfg.ny - cfg.roi)
+        fs.pk[base + i].status = ERROR;
+      else
+        flag = true;
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, flag);
+    __syncwarp();
+    if (flag) fs.run[base + m + __popc(bal & ((1u << lane) - 1u))] = i;
+    m += __popc(bal);
+    __syncwarp();
+  }
+  return m;
+}
+
+// The end of a tail sweep (one warp): recenter the moved peaks, sum the
+// counters (lane i holds counter i of the sweep's steps) and decide the
+// frame's next phase (k_between).  Returns whether another sweep follows.
+template <typename T>
+__device__ inline bool tail_end_sweep(const ModelCfg& cfg, const FrameSet<T>& fs, FrameCtl* c, int base,
+                                      long long fbase, int nrun, long long loc, WarpWS<T>& ws, int lane) {
+  int unconv = 0;
+  for (int r = 0; r < nrun; r++) {
+    const int li = fs.run[base + r];
+    PeakRec rec;
+    load_rec(fs.pk + base + li, rec);
+    if (rec.status != RUNNING) continue;
+    const double dx = rec.p[PX] - rec.xi, dy = rec.p[PY] - rec.yi;
+    if (!((dx < -0.25) || (dx > 1.25) || (dy < -0.25) || (dy > 1.25))) {
+      unconv++;
+      continue;
+    }
+    SplinePos sp = shape_tables(cfg, rec, ws, lane);
+    add_peak(cfg, fs, fbase, rec, sp, ws, -1, lane);
+    __syncwarp();
+    rec.added -= 1;
+    rec.xi = (int)floor(rec.p[PX]);
+    rec.yi = (int)floor(rec.p[PY]);
+    const int chk = base_check(cfg, rec);
+    if (chk) {
+      if (lane == C_LOST || lane == (chk == 1 ? C_MARGIN : C_NEGH)) loc++;
+      rec.status = ERROR;
+    } else {
+      SplinePos s2 = shape_tables(cfg, rec, ws, lane);
+      add_peak(cfg, fs, fbase, rec, s2, ws, +1, lane);
+      rec.added += 1;
+      unconv++;
+    }
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) fs.pk[base + li] = rec;
+    __syncwarp();
+  }
+  if (lane < NCOUNTERS) c->ctr[lane] += loc;
+  const int sweeps = c->sweeps + 1;
+  const bool more = unconv > 0 && sweeps < c->max_sweeps;
+  __syncwarp();
+  if (lane == 0) {
+    c->unconverged = unconv;
+    c->sweeps = sweeps;
+    c->nrun = nrun;
+    c->attempts = 1;
+    c->phase = more ? PH_SWEEP_PENDING : PH_DONE;
+  }
+  __syncwarp();
+  return more;
+}
+
 // One warp (a 32-thread CTA) per frame.  A frame whose fit has made at least
 // one sweep and has at most tail_peaks RUNNING peaks left runs all of its
-// remaining sweeps here, each as k_prepare + k_sweep + k_post would: the
+// remaining sweeps here, each as k_sweep + k_between would: the
 // RUNNING peaks of the previous sweep's run list, in index order, take their
 // LM steps one after another -- the reference's own sequential order
 // (mFitIterateLM multi_fit.c:1072-1349), so every step is unbounded and
@@ -990,7 +1290,7 @@ __global__ void __launch_bounds__(32) k_tail(ModelCfg cfg, FrameSet<T> fs, int t
   const int lane = threadIdx.x;
   const int f = blockIdx.x;
   FrameCtl* c = fs.ctl + f;
-  if (c->phase != PH_SWEEP_PENDING || c->sweeps == 0 || c->unconverged > tail_peaks) return;
+  if (!tail_ready(c, tail_peaks)) return;
   WarpWS<T> ws = warp_ws<T>(smem, cfg, cfg.nroi);
   {
     unsigned short* roi = reinterpret_cast<unsigned short*>(smem + warp_ws_bytes<T>(cfg, cfg.nroi));
@@ -1002,91 +1302,73 @@ __global__ void __launch_bounds__(32) k_tail(ModelCfg cfg, FrameSet<T> fs, int t
   const long long fbase = (long long)f * fs.npix;
   int nrun = c->nrun;
   for (;;) {
-    // run list: the previous run list's RUNNING peaks, in order (k_prepare)
-    int m = 0;
-    for (int k0 = 0; k0 < nrun; k0 += 32) {
-      const int k = k0 + lane;
-      const int i = (k < nrun) ? fs.run[base + k] : -1;
-      bool flag = false;
-      if (i >= 0 && fs.pk[base + i].status == RUNNING) {
-        const PeakRec& q = fs.pk[base + i];
-        if (q.xi < 0 || q.yi < 0 || q.xi >= cfg.nx - cfg.roi || q.yi >= cfg.ny - cfg.roi)
-          fs.pk[base + i].status = ERROR;
-        else
-          flag = true;
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, flag);
-      __syncwarp();
-      if (flag) fs.run[base + m + __popc(bal & ((1u << lane) - 1u))] = i;
-      m += __popc(bal);
-      __syncwarp();
-    }
-    nrun = m;
-    // the steps, one after another in index order (k_sweep)
-    long long loc[NCOUNTERS];
-#pragma unroll
-    for (int i = 0; i < NCOUNTERS; i++) loc[i] = 0;
+    nrun = tail_run_list(cfg, fs, base, nrun, lane);
+    long long loc = 0;
     for (int r = 0; r < nrun; r++) {
       const int li = fs.run[base + r];
       int* sc = fs.stepctr + (size_t)(base + li) * NCOUNTERS;
       if constexpr (G32 >= 0) {
-        g32_prologue<G32>(cfg, fs.pk + base + li, ws, lane);
-        lm_step_g32<G32>(cfg, fs, fbase, fs.pk + base + li, true, 0, ws, sc, lane);
+        warp32::g32_prologue<G32>(cfg, fs.pk + base + li, ws, lane);
+        warp32::lm_step_g32<G32>(cfg, fs, fbase, fs.pk + base + li, true, 0, ws, sc, lane);
       } else {
         lm_step(cfg, fs, fbase, fs.pk + base + li, true, 0, ws, sc, lane);
       }
       __threadfence();
       __syncwarp();
-      if (lane == 0)
-        for (int i = 0; i < NCOUNTERS; i++) loc[i] += sc[i];
+      if (lane < NCOUNTERS) loc += sc[lane];
       __syncwarp();
     }
-    // recenter, count (k_post)
-    int unconv = 0;
+    if (!tail_end_sweep(cfg, fs, c, base, fbase, nrun, loc, ws, lane)) break;
+  }
+}
+
+// k_tail with a team (one CTA) per frame; warp 0 keeps the run list,
+// recentres and counts.
+template <int M>
+__global__ void __launch_bounds__(TEAM) k_tail_team(ModelCfg cfg, FrameSet<float> fs, int tail_peaks) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ TeamCtl tc;
+  __shared__ int s_nrun, s_more;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int f = blockIdx.x;
+  FrameCtl* c = fs.ctl + f;
+  if (!tail_ready(c, tail_peaks)) return;
+  WarpWS<float> ws = g32_team_ws(smem, cfg);
+  // warp 0's view for recentring (the trial tables' memory)
+  WarpWS<float> wr = ws;
+  {
+    unsigned short* roi = reinterpret_cast<unsigned short*>(smem + g32_team_bytes(cfg));
+    for (int i = tid; i < cfg.nroi; i += TEAM) roi[i] = fs.roi_xy[i];
+    ws.roi = roi;
+    wr.tab0 = ws.tab1;
+  }
+  const int base = fs.pk_off[f];
+  const long long fbase = (long long)f * fs.npix;
+  int nrun = c->nrun;
+  for (;;) {
+    if (wid == 0) {
+      const int m = tail_run_list(cfg, fs, base, nrun, lane);
+      if (lane == 0) s_nrun = m;
+    }
+    __syncthreads();
+    nrun = s_nrun;
+    long long loc = 0;   // lane i of warp 0: counter i of this sweep
     for (int r = 0; r < nrun; r++) {
       const int li = fs.run[base + r];
-      PeakRec rec;
-      load_rec(fs.pk + base + li, rec);
-      if (rec.status != RUNNING) continue;
-      const double dx = rec.p[PX] - rec.xi, dy = rec.p[PY] - rec.yi;
-      if (!((dx < -0.25) || (dx > 1.25) || (dy < -0.25) || (dy > 1.25))) {
-        unconv++;
-        continue;
-      }
-      SplinePos sp = shape_tables(cfg, rec, ws, lane);
-      add_peak(cfg, fs, fbase, rec, sp, ws, -1, lane);
-      __syncwarp();
-      rec.added -= 1;
-      rec.xi = (int)floor(rec.p[PX]);
-      rec.yi = (int)floor(rec.p[PY]);
-      const int chk = base_check(cfg, rec);
-      if (chk) {
-        if (lane == 0) {
-          loc[C_LOST]++;
-          loc[chk == 1 ? C_MARGIN : C_NEGH]++;
-        }
-        rec.status = ERROR;
-      } else {
-        SplinePos s2 = shape_tables(cfg, rec, ws, lane);
-        add_peak(cfg, fs, fbase, rec, s2, ws, +1, lane);
-        rec.added += 1;
-        unconv++;
-      }
+      g32_prologue<M, TEAM_WARPS>(cfg, fs, fs.pk + base + li, ws, tid);
+      __syncthreads();
+      lm_step_g32<M>(cfg, fs, fbase, fs.pk + base + li, true, 0, ws, tc,
+                     fs.stepctr + (size_t)(base + li) * NCOUNTERS, tid);
       __threadfence();
-      __syncwarp();
-      if (lane == 0) fs.pk[base + li] = rec;
-      __syncwarp();
+      __syncthreads();
+      if (wid == 0 && lane < NCOUNTERS) loc += reinterpret_cast<const int*>(ws.scratch)[lane];
     }
-    if (lane == 0) {
-      for (int i = 0; i < NCOUNTERS; i++) c->ctr[i] += loc[i];
-      c->unconverged = unconv;
-      c->sweeps += 1;
-      c->nrun = nrun;
-      c->attempts = 1;
-      c->phase = (unconv == 0 || c->sweeps >= c->max_sweeps) ? PH_DONE : PH_SWEEP_PENDING;
+    if (wid == 0) {
+      const bool more = tail_end_sweep(cfg, fs, c, base, fbase, nrun, loc, wr, lane);
+      if (lane == 0) s_more = more;
     }
-    __syncwarp();
-    if (unconv == 0 || *((volatile int*)&c->sweeps) >= c->max_sweeps) break;
+    __syncthreads();
+    if (!s_more) break;
   }
 }
 

@@ -18,19 +18,33 @@ void record_error(const char* msg);
 cudaError_t solve_batch(const double* a, const double* b, int n_sys, int k, double lam, int engine,
                         double* x, int* info, cudaStream_t s);
 
+// Launch shapes of a configuration.
+struct Shapes {
+  int grid = 0;            // sweep CTAs that keep every SM busy (persistent grid), a peak per warp
+  size_t smem = 0;
+  int warps = 0;           // warps of such a CTA
+  int team_grid = 0;       // the same with a peak per CTA (0: no team step, or no room for one)
+  size_t team_smem = 0;
+  size_t cta_smem = 0;     // per-frame CTAs
+  size_t warp_smem = 0;    // warp-per-peak auxiliary CTAs
+};
+
 template <typename T>
 struct Launch {
-  // Set shared-memory limits of the kernels; returns the sweep CTA count
-  // that keeps every SM busy (persistent grid).
-  static cudaError_t configure(const ModelCfg& cfg, int* sweep_grid, size_t* sweep_smem,
-                               size_t* cta_smem, size_t* warp_smem);
-  static cudaError_t prepare(const ModelCfg& cfg, const FrameSet<T>& fs, size_t smem, cudaStream_t s);
-  static cudaError_t sweep(const ModelCfg& cfg, const FrameSet<T>& fs, int grid,
-                           size_t smem, cudaStream_t s);
-  static cudaError_t post(const ModelCfg& cfg, const FrameSet<T>& fs, size_t smem, cudaStream_t s);
+  // Set shared-memory limits of the kernels; returns the launch shapes.
+  static cudaError_t configure(const ModelCfg& cfg, Shapes* sh);
+  // One sweep: a peak per warp, or (team) per CTA.
+  static cudaError_t sweep(const ModelCfg& cfg, const FrameSet<T>& fs, const Shapes& sh, int grid, bool team,
+                           cudaStream_t s);
+  // What lies between sweeps (start_only: of the frames whose fit starts);
+  // the frames' states and the error flag to pinned host memory where poll is
+  // given.
+  static cudaError_t between(const ModelCfg& cfg, const FrameSet<T>& fs, const Shapes& sh, bool start_only,
+                             FramePoll* poll, unsigned* poll_err, cudaStream_t s);
   // The remaining sweeps of every frame with at most tail_peaks RUNNING
-  // peaks left, one warp per frame, in one launch (k_tail).
-  static cudaError_t tail(const ModelCfg& cfg, const FrameSet<T>& fs, int tail_peaks, cudaStream_t s);
+  // peaks left, one warp (or team) per frame, in one launch (k_tail).
+  static cudaError_t tail(const ModelCfg& cfg, const FrameSet<T>& fs, const Shapes& sh, int tail_peaks,
+                          cudaStream_t s);
   static cudaError_t new_image(const FrameSet<T>& fs, const void* img, int bits, int frame0,
                                int nframes, cudaStream_t s);
   static cudaError_t new_background(const FrameSet<T>& fs, const void* bg, int bits, int frame0,

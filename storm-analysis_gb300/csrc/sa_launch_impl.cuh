@@ -17,129 +17,121 @@ static inline int aux_block(const ModelCfg& cfg) { return 32 * aux_warps(cfg); }
 // Shared bytes of the sweep CTA's ROI pixel table (after the workspaces).
 static inline size_t roi_table_bytes(int nroi) { return ((size_t)nroi * 2 + 15) & ~(size_t)15; }
 
-// Warps of a sweep CTA whose dynamic shared memory is smem (configure
-// chooses 4, 3, 2 or 1 so that their workspaces fit).
+// The kernels of a configuration: the FP32 Gaussian models have one
+// instantiation each, everything else shares the generic step.  team_*: the
+// kernels that step a peak per CTA (null: none).
 template <typename T>
-static inline int sweep_warps(const ModelCfg& cfg, size_t smem) {
-  const size_t ws = warp_ws_bytes<T>(cfg, cfg.nroi);
-  const size_t w = (smem - roi_table_bytes(cfg.nroi)) / ws;
-  return w >= 4 ? 4 : (w >= 1 ? (int)w : 1);
-}
+struct Kernels {
+  void (*sweep)(ModelCfg, FrameSet<T>) = k_sweep<T, -1>;
+  void (*tail)(ModelCfg, FrameSet<T>, int) = k_tail<T, -1>;
+  void (*team_sweep)(ModelCfg, FrameSet<T>) = nullptr;
+  void (*team_tail)(ModelCfg, FrameSet<T>, int) = nullptr;
+  size_t team_bytes = 0;
+};
 
-// The sweep kernel of a configuration: the FP32 Gaussian models have one
-// instantiation each, everything else shares the generic step.
 template <typename T>
-void (*sweep_kernel(const ModelCfg& cfg))(ModelCfg, FrameSet<T>) {
+static Kernels<T> kernels(const ModelCfg& cfg) {
+  Kernels<T> k;
   if constexpr (sizeof(T) == 4) {
     if (gauss32<T>(cfg)) {
+      k.team_bytes = g32_team_bytes(cfg);
       switch (cfg.model) {
-        case M_2DFIXED: return k_sweep<T, M_2DFIXED>;
-        case M_2D: return k_sweep<T, M_2D>;
-        case M_3D: return k_sweep<T, M_3D>;
-        default: return k_sweep<T, M_Z>;
+        case M_2DFIXED: k.sweep = k_sweep<T, M_2DFIXED>; k.tail = k_tail<T, M_2DFIXED>; k.team_sweep = k_sweep_team<M_2DFIXED>; k.team_tail = k_tail_team<M_2DFIXED>; break;
+        case M_2D: k.sweep = k_sweep<T, M_2D>; k.tail = k_tail<T, M_2D>; k.team_sweep = k_sweep_team<M_2D>; k.team_tail = k_tail_team<M_2D>; break;
+        case M_3D: k.sweep = k_sweep<T, M_3D>; k.tail = k_tail<T, M_3D>; k.team_sweep = k_sweep_team<M_3D>; k.team_tail = k_tail_team<M_3D>; break;
+        default: k.sweep = k_sweep<T, M_Z>; k.tail = k_tail<T, M_Z>; k.team_sweep = k_sweep_team<M_Z>; k.team_tail = k_tail_team<M_Z>; break;
       }
     }
   }
-  return k_sweep<T, -1>;
+  return k;
 }
 
 template <typename T>
-void (*tail_kernel(const ModelCfg& cfg))(ModelCfg, FrameSet<T>, int) {
-  if constexpr (sizeof(T) == 4) {
-    if (gauss32<T>(cfg)) {
-      switch (cfg.model) {
-        case M_2DFIXED: return k_tail<T, M_2DFIXED>;
-        case M_2D: return k_tail<T, M_2D>;
-        case M_3D: return k_tail<T, M_3D>;
-        default: return k_tail<T, M_Z>;
-      }
-    }
-  }
-  return k_tail<T, -1>;
-}
-
-template <typename T>
-cudaError_t Launch<T>::configure(const ModelCfg& cfg, int* sweep_grid, size_t* sweep_smem,
-                                 size_t* cta_smem, size_t* warp_smem) {
+cudaError_t Launch<T>::configure(const ModelCfg& cfg, Shapes* sh) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   int nsm = 0, max_smem = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  const Kernels<T> k = kernels<T>(cfg);
   const size_t ws = warp_ws_bytes<T>(cfg, cfg.nroi);
   // four warps per sweep CTA, or as many as fit where their workspaces
   // (large ROIs in the FP64 engine, the pupil model) do not
   int wpc = SWEEP_BLOCK / 32;
   while (wpc > 1 && ws * wpc + roi_table_bytes(cfg.nroi) > (size_t)max_smem) wpc--;
-  const size_t s_sweep = ws * wpc + roi_table_bytes(cfg.nroi);
+  sh->warps = wpc;
+  sh->smem = ws * wpc + roi_table_bytes(cfg.nroi);
   const size_t ws0 = warp_ws_bytes<T>(cfg, 0);
   const size_t grid_bytes = (size_t)(cfg.gx * cfg.gy + 1) * sizeof(int);
   const size_t s_cta_ws = ws0 * (size_t)cta_ws_warps(cfg);
-  const size_t s_cta = s_cta_ws > grid_bytes ? s_cta_ws : grid_bytes;
-  const size_t s_aux = ws0 * (size_t)aux_warps(cfg);
-  if (s_sweep > (size_t)max_smem || s_cta > (size_t)max_smem || s_aux > (size_t)max_smem)
-    return cudaErrorInvalidConfiguration;
+  sh->cta_smem = s_cta_ws > grid_bytes ? s_cta_ws : grid_bytes;
+  sh->warp_smem = ws0 * (size_t)aux_warps(cfg);
   // The limit is a property of the kernel, shared by every handle of the
   // process (handles of different models and ROI sizes may run side by
   // side), so it is raised to the device maximum rather than to this
   // handle's need.
-  auto raise_limit = [max_smem](const void* fn) {
+  auto raise_limit = [max_smem](const void* fn, size_t need) {
     cudaFuncAttributes a;
     cudaError_t r = cudaFuncGetAttributes(&a, fn);
     if (r != cudaSuccess) return r;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                max_smem - (int)a.sharedSizeBytes);
+    const int room = max_smem - (int)a.sharedSizeBytes;
+    if (room < (int)need) return cudaErrorInvalidConfiguration;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
   };
-  e = raise_limit((const void*)sweep_kernel<T>(cfg));
-  if (e != cudaSuccess) return e;
-  e = raise_limit((const void*)k_prepare<T>);
-  if (e != cudaSuccess) return e;
-  e = raise_limit((const void*)k_post<T>);
-  if (e != cudaSuccess) return e;
-  e = raise_limit((const void*)tail_kernel<T>(cfg));
-  if (e != cudaSuccess) return e;
-  // the warp-per-peak auxiliary kernels (their workspace is above the
-  // default 48 KB for the FFT PSF model)
-  for (const void* fn : {(const void*)k_newpeaks<T>, (const void*)k_newpeaks_finder<T>, (const void*)k_peak_props<T>,
-                         (const void*)k_set_status<T>}) {
-    e = raise_limit(fn);
+  struct {
+    const void* fn;
+    size_t need;
+  } const all[] = {{(const void*)k.sweep, sh->smem},
+                   {(const void*)k.tail, ws + roi_table_bytes(cfg.nroi)},
+                   {(const void*)k_between<T>, sh->cta_smem},
+                   // the warp-per-peak auxiliary kernels (their workspace is above the
+                   // default 48 KB for the FFT PSF model)
+                   {(const void*)k_newpeaks<T>, sh->warp_smem},
+                   {(const void*)k_newpeaks_finder<T>, sh->warp_smem},
+                   {(const void*)k_peak_props<T>, sh->warp_smem},
+                   {(const void*)k_set_status<T>, sh->warp_smem}};
+  for (const auto& a : all) {
+    e = raise_limit(a.fn, a.need);
     if (e != cudaSuccess) return e;
   }
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel<T>(cfg), 32 * wpc, s_sweep);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.sweep, 32 * wpc, sh->smem);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
-  *sweep_grid = nsm * per_sm;
-  *sweep_smem = s_sweep;
-  *cta_smem = s_cta;
-  *warp_smem = s_aux;
+  sh->grid = nsm * (per_sm < 1 ? 1 : per_sm);
+  // the team kernels, where a team's workspace fits
+  sh->team_smem = k.team_bytes + roi_table_bytes(cfg.nroi);
+  if (k.team_sweep && raise_limit((const void*)k.team_sweep, sh->team_smem) == cudaSuccess &&
+      raise_limit((const void*)k.team_tail, sh->team_smem) == cudaSuccess) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.team_sweep, TEAM, sh->team_smem);
+    if (e != cudaSuccess) return e;
+    sh->team_grid = nsm * per_sm;
+  }
   return cudaSuccess;
 }
 
 template <typename T>
-cudaError_t Launch<T>::prepare(const ModelCfg& cfg, const FrameSet<T>& fs, size_t smem, cudaStream_t s) {
-  k_prepare<T><<<fs.F, CTA_BLOCK, smem, s>>>(cfg, fs);
+cudaError_t Launch<T>::between(const ModelCfg& cfg, const FrameSet<T>& fs, const Shapes& sh, bool start_only,
+                               FramePoll* poll, unsigned* poll_err, cudaStream_t s) {
+  k_between<T><<<fs.F, CTA_BLOCK, sh.cta_smem, s>>>(cfg, fs, start_only ? 1 : 0, poll, poll_err);
   return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t Launch<T>::sweep(const ModelCfg& cfg, const FrameSet<T>& fs, int grid, size_t smem,
+cudaError_t Launch<T>::sweep(const ModelCfg& cfg, const FrameSet<T>& fs, const Shapes& sh, int grid, bool team,
                              cudaStream_t s) {
-  sweep_kernel<T>(cfg)<<<grid, 32 * sweep_warps<T>(cfg, smem), smem, s>>>(cfg, fs);
+  const Kernels<T> k = kernels<T>(cfg);
+  if (team) k.team_sweep<<<grid, TEAM, sh.team_smem, s>>>(cfg, fs);
+  else k.sweep<<<grid, 32 * sh.warps, sh.smem, s>>>(cfg, fs);
   return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t Launch<T>::post(const ModelCfg& cfg, const FrameSet<T>& fs, size_t smem, cudaStream_t s) {
-  k_post<T><<<fs.F, CTA_BLOCK, smem, s>>>(cfg, fs);
-  return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t Launch<T>::tail(const ModelCfg& cfg, const FrameSet<T>& fs, int tail_peaks, cudaStream_t s) {
-  const size_t smem = warp_ws_bytes<T>(cfg, cfg.nroi) + roi_table_bytes(cfg.nroi);
-  tail_kernel<T>(cfg)<<<fs.F, 32, smem, s>>>(cfg, fs, tail_peaks);
+cudaError_t Launch<T>::tail(const ModelCfg& cfg, const FrameSet<T>& fs, const Shapes& sh, int tail_peaks,
+                            cudaStream_t s) {
+  const Kernels<T> k = kernels<T>(cfg);
+  if (sh.team_grid > 0) k.team_tail<<<fs.F, TEAM, sh.team_smem, s>>>(cfg, fs, tail_peaks);
+  else k.tail<<<fs.F, 32, (sh.smem - roi_table_bytes(cfg.nroi)) / sh.warps + roi_table_bytes(cfg.nroi), s>>>(cfg, fs, tail_peaks);
   return cudaGetLastError();
 }
 
