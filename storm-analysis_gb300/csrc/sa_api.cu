@@ -242,6 +242,22 @@ struct Engine {
     return 0;
   }
 
+  // The spline's coefficients [x][y][z][n] (cubic_spline.c:509-522) as the
+  // kernels read them: [quad][z][y][x][4], n = 4 quad + i.
+  std::vector<double> spline_device_layout() const {
+    const int sx = cfg.sx, sy = cfg.sy, sz = spline->type == 1 ? cfg.sz : 1, nq = spline->type == 1 ? 16 : 4;
+    const size_t cells = (size_t)sx * sy * sz;
+    std::vector<double> t(cells * nq * 4);
+    for (int x = 0; x < sx; x++)
+      for (int y = 0; y < sy; y++)
+        for (int z = 0; z < sz; z++) {
+          const double* c = aij_h.data() + (((size_t)x * sy + y) * sz + z) * nq * 4;
+          const size_t cell = ((size_t)z * sy + y) * sx + x;
+          for (int q = 0; q < nq; q++) memcpy(&t[(q * cells + cell) * 4], c + 4 * q, 4 * sizeof(double));
+        }
+    return t;
+  }
+
   // Convert a double host array to the pixel type on the device.
   int upload_t(void** dst, const double* src, size_t n) {
     dfree(*dst);
@@ -310,7 +326,10 @@ struct Engine {
     if (!d_rqe) {
       if (upload_t(&d_rqe, rqe_h.data(), npix)) return -1;
       if (upload_t(&d_scmos, scmos_h.data(), npix)) return -1;
-      if (!aij_h.empty() && upload_t(&d_aij, aij_h.data(), aij_h.size())) return -1;
+      if (!aij_h.empty()) {
+        const std::vector<double> t = spline ? spline_device_layout() : std::vector<double>();
+        if (upload_t(&d_aij, t.empty() ? aij_h.data() : t.data(), aij_h.size())) return -1;
+      }
       // the FFT and pupil models' tables (FP64: d_aij holds them as doubles)
       if (cfg.model == M_FFT || cfg.model == M_PUPIL) cfg.fft = static_cast<const double*>(d_aij);
       CK(cudaMalloc(&d_roi, roi_xy.size() * sizeof(unsigned short)));

@@ -1125,11 +1125,11 @@ __device__ __forceinline__ void g32_contrib(const float* tab, int ts, ff H, ff B
 // offset uses xoff as the reference does (:979).
 template <typename T>
 __device__ inline void gauss_tables(const ModelCfg& cfg, const double* p, int xi, int yi,
-                                    WarpWS<T>& ws, int lane) {
+                                    WarpWS<T>& ws, int lane, int stride = 32) {
   const double xo = -(p[PX] - (double)xi) - cfg.xoff;
   const double yo = -(p[PY] - (double)yi) - cfg.xoff;
   const T wx = (T)p[PXW], wy = (T)p[PYW];
-  for (int i = lane; i < cfg.roi; i += 32) {
+  for (int i = lane; i < cfg.roi; i += stride) {
     T tx = (T)((double)i + xo);
     T ty = (T)((double)i + yo);
     ws.xt[i] = tx;
@@ -1187,11 +1187,11 @@ __device__ __forceinline__ ff ff_pow(ff v, int e) {
 // (FP64 oracle with 1e-8 relative noise on the value; 1e-9: 0.1 %).
 template <typename T>
 __device__ inline void spline_value_monomials(const ModelCfg& cfg, const SplinePos& s, WarpWS<T>& ws,
-                                              int lane) {
+                                              int lane, int stride = 32) {
   const bool three = (cfg.model == M_SPLINE3D);
   const ff x = ff_from_double(clamp01(s.xd)), y = ff_from_double(clamp01(s.yd));
   const ff z = ff_from_double(three ? clamp01(s.zd) : 0.0);
-  for (int id = lane; id < (three ? 64 : 16); id += 32) {
+  for (int id = lane; id < (three ? 64 : 16); id += stride) {
     const int a = three ? (id >> 4) : (id >> 2);
     const int b = three ? ((id >> 2) & 3) : (id & 3);
     const int c = three ? (id & 3) : 0;
@@ -1203,11 +1203,11 @@ __device__ inline void spline_value_monomials(const ModelCfg& cfg, const SplineP
 
 template <typename T>
 __device__ inline void spline_tables(const ModelCfg& cfg, const SplinePos& s, WarpWS<T>& ws,
-                                     int lane) {
+                                     int lane, int stride = 32) {
   const T x = (T)clamp01(s.xd), y = (T)clamp01(s.yd);
   if (cfg.model == M_SPLINE3D) {
     const T z = (T)clamp01(s.zd);
-    for (int id = lane; id < 64; id += 32) {
+    for (int id = lane; id < 64; id += stride) {
       const int a = id >> 4, b = (id >> 2) & 3, c = id & 3;
       const T px = pw(x, a), py = pw(y, b), pz = pw(z, c);
       if (sizeof(T) != 4) ws.ext[id] = mul_rn(mul_rn(px, py), pz);
@@ -1217,7 +1217,7 @@ __device__ inline void spline_tables(const ModelCfg& cfg, const SplinePos& s, Wa
       ws.eyt[64 + id] = (c > 0) ? mul_rn(mul_rn(px, py), mul_rn((T)c, pw(z, c - 1))) : (T)0;
     }
   } else {
-    for (int id = lane; id < 16; id += 32) {
+    for (int id = lane; id < 16; id += stride) {
       const int a = id >> 2, b = id & 3;
       const T px = pw(x, a), py = pw(y, b);
       if (sizeof(T) != 4) ws.ext[id] = mul_rn(px, py);
@@ -1225,52 +1225,79 @@ __device__ inline void spline_tables(const ModelCfg& cfg, const SplinePos& s, Wa
       ws.eyt[id] = (b > 0) ? mul_rn(px, mul_rn((T)b, pw(y, b - 1))) : (T)0;
     }
   }
-  if constexpr (sizeof(T) == 4) spline_value_monomials(cfg, s, ws, lane);
+  if constexpr (sizeof(T) == 4) spline_value_monomials(cfg, s, ws, lane, stride);
 }
 
 __device__ __forceinline__ int clampi(int v, int hi_excl) {
   return v < 0 ? 0 : (v >= hi_excl ? hi_excl - 1 : v);
 }
 
-// Spline cell base (fAt3D index clamps, cubic_spline.c:509-522).
-template <typename T>
-__device__ __forceinline__ const T* spline_cell(const ModelCfg& cfg, const T* aij, int zc, int yc,
-                                                int xc) {
+// Spline coefficients on the device (spline_device_layout, sa_api.cu): four
+// consecutive ones of every cell together, cells with x fastest, so that the
+// pixels of a ROI row -- neighbouring lanes -- read neighbouring quads.  In the
+// reference's order (a cell's 64 coefficients together) every load of a warp
+// touched 32 lines.  Index clamps as fAt3D, cubic_spline.c:509-522.
+__device__ __forceinline__ int spline_cell(const ModelCfg& cfg, int zc, int yc, int xc) {
   xc = clampi(xc, cfg.sx);
   yc = clampi(yc, cfg.sy);
-  if (cfg.model == M_SPLINE3D) {
-    zc = clampi(zc, cfg.sz);
-    return aij + ((size_t)xc * (cfg.sy * cfg.sz) + (size_t)yc * cfg.sz + zc) * 64;
-  }
-  return aij + ((size_t)xc * cfg.sy + yc) * 16;
+  if (cfg.model != M_SPLINE3D) return yc * cfg.sx + xc;
+  return (clampi(zc, cfg.sz) * cfg.sy + yc) * cfg.sx + xc;
+}
+__device__ __forceinline__ int spline_quads(const ModelCfg& cfg) { return cfg.model == M_SPLINE3D ? 16 : 4; }
+__device__ __forceinline__ int spline_cells(const ModelCfg& cfg) {
+  return cfg.sx * cfg.sy * (cfg.model == M_SPLINE3D ? cfg.sz : 1);
+}
+__device__ __forceinline__ void spline_quad(const float* aij, size_t at, float (&c)[4]) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(aij) + at);
+  c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
+}
+__device__ __forceinline__ void spline_quad(const double* aij, size_t at, double (&c)[4]) {
+  const double2 u = __ldg(reinterpret_cast<const double2*>(aij) + 2 * at);
+  const double2 v = __ldg(reinterpret_cast<const double2*>(aij) + 2 * at + 1);
+  c[0] = u.x; c[1] = u.y; c[2] = v.x; c[3] = v.y;
 }
 
 // Dot of a spline cell with one of the monomial tables, in a fixed order.
 template <typename T>
-__device__ __forceinline__ T spline_dot(const T* c, const T* tab, int n) {
+__device__ __forceinline__ T spline_dot(const ModelCfg& cfg, const T* aij, int cell, const T* tab) {
+  const int nq = spline_quads(cfg);
+  const size_t nc = spline_cells(cfg);
   T acc = (T)0;
-#pragma unroll 8
-  for (int i = 0; i < n; i++) acc = fma_rn(__ldg(c + i), tab[i], acc);
+#pragma unroll 2
+  for (int q = 0; q < nq; q++) {
+    T c[4];
+    spline_quad(aij, q * nc + cell, c);
+#pragma unroll
+    for (int i = 0; i < 4; i++) acc = fma_rn(c[i], tab[4 * q + i], acc);
+  }
   return acc;
 }
 
-// FP32 engine: the spline's value at ROI pixel (rx, ry) as float-float: a
-// compensated dot (Ogita, Rump and Oishi's Dot2, with the float-float
-// monomials' lo words folded into the error sum) of the cell's FP32
-// coefficients with the value monomials of spline_value_monomials.
+// FP32 engine: one coefficient's step of the spline's value as a compensated
+// dot (Ogita, Rump and Oishi's Dot2, with the float-float monomials' lo words
+// folded into the error sum); (hi, err) is closed by fast_two_sum.
+__device__ __forceinline__ void spline_value_acc(float ci, float mh, float ml, float& hi, float& err) {
+  const float p = __fmul_rn(ci, mh);
+  const float pe = __fmaf_rn(ci, mh, -p);
+  const ff t = two_sum(hi, p);
+  hi = t.h;
+  err = __fmaf_rn(ci, ml, __fadd_rn(err, __fadd_rn(t.l, pe)));
+}
+
+// FP32 engine: the spline's value at ROI pixel (rx, ry) as float-float, from
+// the cell's FP32 coefficients and the value monomials of
+// spline_value_monomials.
 __device__ __forceinline__ ff spline_value_ff(const ModelCfg& cfg, const float* aij, const WarpWS<float>& ws,
                                               const SplinePos& s, int rx, int ry) {
-  const int nc = (cfg.model == M_SPLINE3D) ? 64 : 16;
-  const float* c = spline_cell(cfg, aij, s.zi, ry + s.ys, rx + s.xs);
+  const int nq = spline_quads(cfg), cell = spline_cell(cfg, s.zi, ry + s.ys, rx + s.xs);
+  const size_t nc = spline_cells(cfg);
   float hi = 0.0f, err = 0.0f;
-#pragma unroll 8
-  for (int i = 0; i < nc; i++) {
-    const float ci = __ldg(c + i);
-    const float p = __fmul_rn(ci, ws.ext[i]);
-    const float pe = __fmaf_rn(ci, ws.ext[i], -p);
-    const ff t = two_sum(hi, p);
-    hi = t.h;
-    err = __fmaf_rn(ci, ws.yt[i], __fadd_rn(err, __fadd_rn(t.l, pe)));
+#pragma unroll 2
+  for (int q = 0; q < nq; q++) {
+    float c[4];
+    spline_quad(aij, q * nc + cell, c);
+#pragma unroll
+    for (int i = 0; i < 4; i++) spline_value_acc(c[i], ws.ext[4 * q + i], ws.yt[4 * q + i], hi, err);
   }
   return fast_two_sum(hi, err);
 }
@@ -1301,8 +1328,15 @@ __device__ __forceinline__ void spl32_contrib(ff psf, ff H, ff BG, float rq, flo
 
 constexpr double SA_PI = 3.14159265358979323846;   // the reference's M_PI
 
-template <typename T>
-__device__ inline void fft_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<T>& ws, int lane) {
+// By stride threads (a warp, or more of a team), sync their barrier; deriv
+// false: without the arrays of the derivatives (Cz, Dy, Dz).
+struct WarpSync {
+  __device__ __forceinline__ void operator()() const { __syncwarp(); }
+};
+
+template <typename T, typename Sync = WarpSync>
+__device__ inline void fft_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<T>& ws, int lane, bool deriv = true,
+                                  int stride = 32, const Sync& sync = Sync()) {
   const int nx = cfg.sx, ny = cfg.sy, nz = cfg.sz;
   const FFTLayout L = fft_layout(nx, ny, nz);
   const int nk = L.nk;
@@ -1319,7 +1353,7 @@ __device__ inline void fft_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<
   // entry k is cos / sin of t1 * m with m = k up to size/2 (the sine kept
   // positive at size/2, the reference loop's second write) and m = size - k
   // with the sine negated above it
-  for (int i = lane; i < nk + ny + nz; i += 32) {
+  for (int i = lane; i < nk + ny + nz; i += stride) {
     int size, k;
     double d;
     double* out;
@@ -1341,11 +1375,11 @@ __device__ inline void fft_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<
     out[0] = re;
     out[1] = im;
   }
-  __syncwarp();
+  sync();
   const double* Wt = cfg.fft + L.w;
   const double* Ez = cfg.fft + L.ez;
   const double* dkz = cfg.fft + L.dkz;
-  for (int q = lane; q < ny * nk; q += 32) {
+  for (int q = lane; q < ny * nk; q += stride) {
     const int ky = q / nk, kx = q - ky * nk;
     const double syr = syv[2 * ky], syi = syv[2 * ky + 1], sxr = sxv[2 * kx], sxi = sxv[2 * kx + 1];
     double cr = 0.0, ci = 0.0, czr = 0.0, czi = 0.0;
@@ -1363,19 +1397,23 @@ __device__ inline void fft_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<
       const double pr = r2 * er - c2 * ei, pi = r2 * ei + c2 * er;
       cr += pr;
       ci += pi;
-      const double dk = __ldg(dkz + kz);
-      czr += pi * dk;
-      czi -= pr * dk;
+      if (deriv) {
+        const double dk = __ldg(dkz + kz);
+        czr += pi * dk;
+        czi -= pr * dk;
+      }
     }
     C[2 * q] = cr;
     C[2 * q + 1] = ci;
-    Cz[2 * q] = czr;
-    Cz[2 * q + 1] = czi;
+    if (deriv) {
+      Cz[2 * q] = czr;
+      Cz[2 * q + 1] = czi;
+    }
   }
-  __syncwarp();
+  sync();
   const double* Ey = cfg.fft + L.ey;
   const double* dky = cfg.fft + L.dky;
-  for (int q = lane; q < ny * nk; q += 32) {
+  for (int q = lane; q < ny * nk; q += stride) {
     const int y = q / nk, kx = q - y * nk;
     double dr = 0.0, di = 0.0, dyr = 0.0, dyi = 0.0, dzr = 0.0, dzi = 0.0;
     for (int ky = 0; ky < ny; ky++) {
@@ -1385,19 +1423,23 @@ __device__ inline void fft_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<
       const double pr = ar * er - ai * ei, pi = ar * ei + ai * er;
       dr += pr;
       di += pi;
-      const double dk = __ldg(dky + ky);
-      dyr += pi * dk;
-      dyi -= pr * dk;
-      const double zr = Cz[c], zi = Cz[c + 1];
-      dzr += zr * er - zi * ei;
-      dzi += zr * ei + zi * er;
+      if (deriv) {
+        const double dk = __ldg(dky + ky);
+        dyr += pi * dk;
+        dyi -= pr * dk;
+        const double zr = Cz[c], zi = Cz[c + 1];
+        dzr += zr * er - zi * ei;
+        dzi += zr * ei + zi * er;
+      }
     }
     Dm[2 * q] = dr;
     Dm[2 * q + 1] = di;
-    Dy[2 * q] = dyr;
-    Dy[2 * q + 1] = dyi;
-    Dz[2 * q] = dzr;
-    Dz[2 * q + 1] = dzi;
+    if (deriv) {
+      Dy[2 * q] = dyr;
+      Dy[2 * q + 1] = dyi;
+      Dz[2 * q] = dzr;
+      Dz[2 * q + 1] = dzi;
+    }
   }
 }
 
@@ -1448,19 +1490,24 @@ __device__ inline double fft_pixel(const ModelCfg& cfg, const double* fw, int rx
 // pfitInitialize checks on the host).
 // ---------------------------------------------------------------------------
 
-template <typename T>
-__device__ inline void pupil_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<T>& ws, int lane,
-                                    bool deriv) {
+// By stride threads (a warp, or more of a team, each warp with its own three
+// row buffers: the first warp's are in the workspace, the others' at rows),
+// sync their barrier.
+template <typename T, typename Sync = WarpSync>
+__device__ inline void pupil_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<T>& ws, int tid, bool deriv,
+                                    int stride = 32, double* rows = nullptr, const Sync& sync = Sync()) {
+  const int lane = tid & 31, wid = tid >> 5;
   const int n = cfg.sx, m = n / 2, m1 = m + 1;
   const int hb = pupil_band_rows(n, cfg.sz);
   const PupilLayout L = pupil_layout(n);
   double* B = ws.fw;             // row i of the band at (i - i_lo) * n
   double* By = B + 2 * hb * n;
   double* Bz = By + 2 * hb * n;
-  double* rw = Bz + 2 * hb * n;  // the translated pupil function's row i (complex)
+  double* row0 = Bz + 2 * hb * n;
+  double* rw = wid == 0 ? row0 : rows + (wid - 1) * 6 * n;   // the translated pupil function's row i (complex)
   double* rwy = rw + 2 * n;      // ... times -i ky
   double* rwz = rwy + 2 * n;     // ... times -i kz
-  double* sxv = rwz + 2 * n;     // x shift per first index (complex)
+  double* sxv = row0 + 6 * n;    // x shift per first index (complex)
   double* syv = sxv + 2 * n;     // y shift per second index (complex)
   double* szt = syv + 2 * n;     // z shift per pie-slice offset [m+1][m+1] (complex)
   const double* E = cfg.fft + L.e;
@@ -1472,7 +1519,7 @@ __device__ inline void pupil_tables(const ModelCfg& cfg, const PeakRec& w, WarpW
   // pfitCalcPeakShape :148-150
   const double dx = w.p[PX] - (double)w.xi, dy = w.p[PY] - (double)w.yi, dz = w.p[PZ];
   // shift vectors, pfnTranslate :453-463 (both from kx's first column)
-  for (int i = lane; i < 2 * n; i += 32) {
+  for (int i = tid; i < 2 * n; i += stride) {
     const int j = i < n ? i : i - n;
     const double dd = __ldg(KX + j) * (i < n ? dx : dy);
     double sv, cv;
@@ -1482,7 +1529,7 @@ __device__ inline void pupil_tables(const ModelCfg& cfg, const PeakRec& w, WarpW
     o[1] = -sv;
   }
   // z shift over the pie slice, :475-486 (with -dz); symmetric in (a, b)
-  for (int q = lane; q < m1 * m1; q += 32) {
+  for (int q = tid; q < m1 * m1; q += stride) {
     const int a = q / m1, b = q - a * m1;
     if (a <= b) {
       const double dd = -__ldg(KZS + q) * dz;
@@ -1494,9 +1541,9 @@ __device__ inline void pupil_tables(const ModelCfg& cfg, const PeakRec& w, WarpW
       szt[2 * (b * m1 + a) + 1] = -sv;
     }
   }
-  __syncwarp();
+  sync();
   const int i_lo = (int)__ldg(cfg.fft + L.band), i_hi = (int)__ldg(cfg.fft + L.band + 1);
-  for (int i = i_lo; i <= i_hi; i++) {
+  for (int i = i_lo + wid; i <= i_hi; i += stride / 32) {
     const double xr = sxv[2 * i], xc = sxv[2 * i + 1];
     const int oa = abs(i - m) * m1;
     const int k_lo = (int)__ldg(cfg.fft + L.rng + 2 * i), k_hi = (int)__ldg(cfg.fft + L.rng + 2 * i + 1);
@@ -1616,9 +1663,7 @@ __device__ __forceinline__ T psf_at(const ModelCfg& cfg, const T* aij, const War
   if constexpr (sizeof(T) == 4) {
     return spline_value_ff(cfg, aij, ws, s, rx, ry).h;
   } else {
-    const int nc = (cfg.model == M_SPLINE3D) ? 64 : 16;
-    const T* c = spline_cell(cfg, aij, s.zi, ry + s.ys, rx + s.xs);
-    return spline_dot(c, ws.ext, nc);
+    return spline_dot(cfg, aij, spline_cell(cfg, s.zi, ry + s.ys, rx + s.xs), ws.ext);
   }
 }
 
@@ -1731,7 +1776,7 @@ __device__ __forceinline__ int check_for(const ModelCfg& cfg, int model, PeakRec
 
 // Prepare the shape tables of peak w (all lanes) and return its spline
 // position (unused for Gaussians).  deriv false: only the shape will be
-// read (the pupil model then skips its derivative sums).
+// read (the FFT and pupil models then skip their derivative sums).
 template <typename T>
 __device__ inline SplinePos shape_tables(const ModelCfg& cfg, const PeakRec& w, WarpWS<T>& ws,
                                          int lane, bool deriv = true) {
@@ -1739,7 +1784,7 @@ __device__ inline SplinePos shape_tables(const ModelCfg& cfg, const PeakRec& w, 
   if (is_fft(cfg.model)) {
     s.xs = s.ys = s.zi = 0;
     s.xd = s.yd = s.zd = 0.0;
-    fft_tables(cfg, w, ws, lane);
+    fft_tables(cfg, w, ws, lane, deriv);
   } else if (is_pupil(cfg.model)) {
     s.xs = s.ys = s.zi = 0;
     s.xd = s.yd = s.zd = 0.0;
@@ -1831,14 +1876,20 @@ __device__ __forceinline__ void jt_row(const ModelCfg& cfg, const T* aij, const 
       break;
     }
     case M_SPLINE3D: {
-      const T* c = spline_cell(cfg, aij, s.zi, ry + s.ys, rx + s.xs);
+      const int cell = spline_cell(cfg, s.zi, ry + s.ys, rx + s.xs);
+      const size_t nc = spline_cells(cfg);
       T dx = (T)0, dy = (T)0, dz = (T)0;
-#pragma unroll 8
-      for (int i = 0; i < 64; i++) {
-        const T ci = __ldg(c + i);
-        dx = fma_rn(ci, ws.ext[64 + i], dx);
-        dy = fma_rn(ci, ws.eyt[i], dy);
-        dz = fma_rn(ci, ws.eyt[64 + i], dz);
+#pragma unroll 2
+      for (int q = 0; q < 16; q++) {
+        T c[4];
+        spline_quad(aij, q * nc + cell, c);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int i = 4 * q + j;
+          dx = fma_rn(c[j], ws.ext[64 + i], dx);
+          dy = fma_rn(c[j], ws.eyt[i], dy);
+          dz = fma_rn(c[j], ws.eyt[64 + i], dz);
+        }
       }
       jt[0] = rq * psf;
       jt[1] = -rq * h * dx;
@@ -1848,13 +1899,18 @@ __device__ __forceinline__ void jt_row(const ModelCfg& cfg, const T* aij, const 
       break;
     }
     default: {  // M_SPLINE2D
-      const T* c = spline_cell(cfg, aij, 0, ry + s.ys, rx + s.xs);
+      const int cell = spline_cell(cfg, 0, ry + s.ys, rx + s.xs);
+      const size_t nc = spline_cells(cfg);
       T dx = (T)0, dy = (T)0;
-#pragma unroll 8
-      for (int i = 0; i < 16; i++) {
-        const T ci = __ldg(c + i);
-        dx = fma_rn(ci, ws.ext[64 + i], dx);
-        dy = fma_rn(ci, ws.eyt[i], dy);
+#pragma unroll 2
+      for (int q = 0; q < 4; q++) {
+        T c[4];
+        spline_quad(aij, q * nc + cell, c);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          dx = fma_rn(c[j], ws.ext[64 + 4 * q + j], dx);
+          dy = fma_rn(c[j], ws.eyt[4 * q + j], dy);
+        }
       }
       jt[0] = rq * psf;
       jt[1] = -rq * h * dx;
@@ -1881,7 +1937,8 @@ __device__ __forceinline__ void jt_row(const ModelCfg& cfg, const T* aij, const 
 
 template <typename T>
 __device__ inline void diff_tables(const ModelCfg& cfg, const PeakRec& w0, const PeakRec& w1,
-                                   const SplinePos& s0, const SplinePos& s1, WarpWS<T>& ws, int lane) {
+                                   const SplinePos& s0, const SplinePos& s1, WarpWS<T>& ws, int lane,
+                                   int stride = 32) {
   if (!is_spline(cfg.model)) {
     // per-warp scalars from the FP64 parameters (differences taken in FP64)
     const float xo0 = (float)(-(w0.p[PX] - (double)w0.xi) - cfg.xoff);
@@ -1905,7 +1962,7 @@ __device__ inline void diff_tables(const ModelCfg& cfg, const PeakRec& w0, const
     const T X0 = (T)x0, X1 = (T)x1, Y0 = (T)y0, Y1 = (T)y1, Z0 = (T)z0, Z1 = (T)z1;
     const bool three = (cfg.model == M_SPLINE3D);
     const int nmono = three ? 64 : 16;
-    for (int id = lane; id < nmono; id += 32) {
+    for (int id = lane; id < nmono; id += stride) {
       const int a = three ? (id >> 4) : (id >> 2);
       const int b = three ? ((id >> 2) & 3) : (id & 3);
       const int c = three ? (id & 3) : 0;
@@ -1932,17 +1989,9 @@ __device__ __forceinline__ void psf_and_delta(const ModelCfg& cfg, const T* aij,
     dpsf = ey0 * dex + dey * (ex0 + dex);
     return;
   }
-  const int nc = (cfg.model == M_SPLINE3D) ? 64 : 16;
-  const T* c = spline_cell(cfg, aij, s.zi, ry + s.ys, rx + s.xs);
-  T acc = (T)0, dacc = (T)0;
-#pragma unroll 8
-  for (int i = 0; i < nc; i++) {
-    const T ci = __ldg(c + i);
-    acc = fma_rn(ci, ws.ext[i], acc);
-    dacc = fma_rn(ci, ws.xt[i], dacc);
-  }
-  psf = acc;
-  dpsf = dacc;
+  const int cell = spline_cell(cfg, s.zi, ry + s.ys, rx + s.xs);
+  psf = spline_dot(cfg, aij, cell, ws.ext);
+  dpsf = spline_dot(cfg, aij, cell, ws.xt);
 }
 
 // ---------------------------------------------------------------------------
