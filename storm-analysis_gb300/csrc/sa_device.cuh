@@ -2183,6 +2183,19 @@ __device__ __forceinline__ Q2 q_sub(Q2 a, Q2 b) {
   return r;
 }
 
+template <typename T>
+__device__ __forceinline__ T ic_store(int c) {
+  // FP32 keeps 1/count and multiplies; FP64 keeps the count and divides as
+  // the reference does (multi_fit.c:143).
+  if (sizeof(T) == 4) return c > 0 ? (T)1 / (T)c : (T)0;
+  return (T)c;
+}
+template <typename T>
+__device__ __forceinline__ T bg_div(T b, T ic) {
+  if (sizeof(T) == 4) return b * ic;
+  return b / ic;
+}
+
 // Add (sign +1) or subtract (sign -1) a peak's contribution over its ROI
 // with integer atomics (mFitAddPeak multi_fit.c:28-57, mFitSubtractPeak
 // :1894-1922).  The shape tables of w must be in the workspace.  By a warp, or

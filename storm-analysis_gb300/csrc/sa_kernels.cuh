@@ -19,6 +19,7 @@
 
 #include <cstddef>
 #include "sa_g32w.cuh"
+#include "sa_team.cuh"
 
 namespace sa {
 
@@ -68,19 +69,6 @@ __device__ __forceinline__ void load_rec(const PeakRec* src, PeakRec& dst) {
 // ---------------------------------------------------------------------------
 // the LM step of one peak (one warp)
 // ---------------------------------------------------------------------------
-
-template <typename T>
-__device__ __forceinline__ T ic_store(int c) {
-  // FP32 keeps 1/count and multiplies; FP64 keeps the count and divides as
-  // the reference does (multi_fit.c:143).
-  if (sizeof(T) == 4) return c > 0 ? (T)1 / (T)c : (T)0;
-  return (T)c;
-}
-template <typename T>
-__device__ __forceinline__ T bg_div(T b, T ic) {
-  if (sizeof(T) == 4) return b * ic;
-  return b / ic;
-}
 
 // Load the base pixel state (fit image without this peak) at anchor (ax, ay).
 template <typename T>
@@ -782,18 +770,87 @@ __device__ inline int grab_rank(const FrameSet<T>& fs, int& f, int lane) {
   return -1;
 }
 
+// The team steps.  THREADS of a CTA, CTAs per SM to compile for, the
+// workspace and the step's parts.  PRO: threads of the prologue (the last
+// warp waits for the predecessors meanwhile).
 template <int M>
-__global__ void __launch_bounds__(TEAM, 8) k_sweep_team(ModelCfg cfg, FrameSet<float> fs) {
-  extern __shared__ __align__(16) char smem[];
-  __shared__ TeamCtl tc;
-  const int epoch = __ldcg(fs.epoch);
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  WarpWS<float> ws = g32_team_ws(smem, cfg);
-  {
-    unsigned short* roi = reinterpret_cast<unsigned short*>(smem + g32_team_bytes(cfg));
-    for (int i = tid; i < cfg.nroi; i += TEAM) roi[i] = fs.roi_xy[i];
+struct StepG32 {
+  using T = float;
+  using WS = WarpWS<float>;
+  static constexpr int THREADS = TEAM, MIN_CTAS = 8;
+  __host__ __device__ static size_t bytes(const ModelCfg& cfg) { return g32_team_bytes(cfg); }
+  __device__ static WS workspace(char* smem, const ModelCfg& cfg) { return g32_team_ws(smem, cfg); }
+  __device__ static void pixel_tables(const ModelCfg& cfg, const FrameSet<T>& fs, char* smem, WS& ws, unsigned short* roi) {
     ws.roi = roi;
   }
+  // warp 0's view for recentering (the trial tables' memory)
+  __device__ static WarpWS<T> aux(const WS& ws) {
+    WarpWS<T> w = ws;
+    w.tab0 = ws.tab1;
+    return w;
+  }
+  template <int PRO>
+  __device__ static void prologue(const ModelCfg& cfg, const FrameSet<T>& fs, const PeakRec* rec, WS& ws, int tid) {
+    g32_prologue<M, PRO / 32>(cfg, fs, rec, ws, tid);
+  }
+  __device__ static bool step(const ModelCfg& cfg, const FrameSet<T>& fs, long long fbase, PeakRec* rec, bool unbounded,
+                              int dil, WS& ws, TeamCtl& tc, int* ctr, int tid) {
+    return lm_step_g32<M>(cfg, fs, fbase, rec, unbounded, dil, ws, tc, ctr, tid);
+  }
+  __device__ static WarpWS<T>& view(WS& ws) { return ws; }
+};
+
+// The generic step; the model is one of a group (the compiler drops the
+// others' code): 0 Gaussians, 1 splines, 2 FFT PSF, 3 pupil function.
+template <typename T_, int GROUP>
+struct StepTeam {
+  using T = T_;
+  using WS = TeamWS<T>;
+  // An FP64 Gaussian ROI is one pixel per thread of four warps; the others are
+  // several times as large, and their tables want every warp.
+  static constexpr int THREADS = GROUP == 0 ? 128 : 256, MIN_CTAS = GROUP == 0 ? 4 : 2;
+  __host__ __device__ static size_t bytes(const ModelCfg& cfg) { return team_ws_bytes<T>(cfg, THREADS); }
+  __device__ static WS workspace(char* smem, const ModelCfg& cfg) {
+    const int m = cfg.model;
+    __builtin_assume(GROUP == 0 ? m <= M_Z : GROUP == 1 ? (m == M_SPLINE2D || m == M_SPLINE3D) : m == (GROUP == 2 ? M_FFT : M_PUPIL));
+    return team_ws<T>(smem, cfg, THREADS);
+  }
+  __device__ static void pixel_tables(const ModelCfg& cfg, const FrameSet<T>& fs, char* smem, WS& ws, unsigned short* roi) {
+    ws.b.roi = roi;
+    unsigned short* inv = const_cast<unsigned short*>(ws.inv);
+    for (int i = threadIdx.x; i < cfg.nroi; i += THREADS) {
+      int rx, ry;
+      roi_rc(fs.roi_xy, i, rx, ry);
+      inv[ry * cfg.roi + rx] = (unsigned short)i;
+    }
+  }
+  __device__ static WarpWS<T> aux(const WS& ws) { return ws.b; }
+  template <int PRO>
+  __device__ static void prologue(const ModelCfg& cfg, const FrameSet<T>& fs, const PeakRec* rec, WS& ws, int tid) {
+    team_prologue<PRO>(cfg, fs, rec, ws, tid);
+  }
+  __device__ static bool step(const ModelCfg& cfg, const FrameSet<T>& fs, long long fbase, PeakRec* rec, bool unbounded,
+                              int dil, WS& ws, TeamCtl& tc, int* ctr, int tid) {
+    return team_step<THREADS>(cfg, fs, fbase, rec, unbounded, dil, ws, tc, ctr, tid);
+  }
+  __device__ static WarpWS<T>& view(WS& ws) { return ws.b; }
+};
+
+template <typename S>
+__global__ void __launch_bounds__(S::THREADS, S::MIN_CTAS)
+    k_sweep_team(const __grid_constant__ ModelCfg cfg, const __grid_constant__ FrameSet<typename S::T> fs) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ TeamCtl tc;
+  constexpr int PRO = S::THREADS - 32;
+  const int epoch = __ldcg(fs.epoch);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  typename S::WS ws = S::workspace(smem, cfg);
+  {
+    unsigned short* roi = reinterpret_cast<unsigned short*>(smem + S::bytes(cfg));
+    for (int i = tid; i < cfg.nroi; i += S::THREADS) roi[i] = fs.roi_xy[i];
+    S::pixel_tables(cfg, fs, smem, ws, roi);
+  }
+  const WarpWS<typename S::T>& v = S::view(ws);
   int fcur = blockIdx.x % fs.F;   // warp 0's
   for (;;) {
     if (wid == 0) {
@@ -812,10 +869,10 @@ __global__ void __launch_bounds__(TEAM, 8) k_sweep_team(ModelCfg cfg, FrameSet<f
     const int f = tc.f, li = tc.li;
     const int base = fs.pk_off[f];
     FrameCtl* c = fs.ctl + f;
-    // warp 3 waits for the step's predecessors while the others compute what
-    // the step needs of its own record
-    if (wid < 3) {
-      g32_prologue<M, 3>(cfg, fs, fs.pk + base + li, ws, tid);
+    // the last warp waits for the step's predecessors while the others
+    // compute what the step needs of its own record
+    if (tid < PRO) {
+      S::template prologue<PRO>(cfg, fs, fs.pk + base + li, ws, tid);
     } else {
       const int start = c->start, dil = c->dil, nb = c->n_barrier;
       const unsigned a0 = fs.anchor0[base + r];
@@ -832,7 +889,7 @@ __global__ void __launch_bounds__(TEAM, 8) k_sweep_team(ModelCfg cfg, FrameSet<f
         tc.nb = nb;
       }
     }
-    // No fence before the step: warp 3's acquire loads of the dependencies'
+    // No fence before the step: the last warp's acquire loads of the dependencies'
     // done flags, and this barrier, order the step's reads after the
     // predecessors' writes.
     __syncthreads();
@@ -840,8 +897,8 @@ __global__ void __launch_bounds__(TEAM, 8) k_sweep_team(ModelCfg cfg, FrameSet<f
     if (go == 0) return;
     bool esc = false;
     if (go == 1)
-      esc = lm_step_g32<M>(cfg, fs, (long long)f * fs.npix, fs.pk + base + li, tc.barrier != 0, tc.dil, ws, tc,
-                           fs.stepctr + (size_t)(base + li) * NCOUNTERS, tid);
+      esc = S::step(cfg, fs, (long long)f * fs.npix, fs.pk + base + li, tc.barrier != 0, tc.dil, ws, tc,
+                    fs.stepctr + (size_t)(base + li) * NCOUNTERS, tid);
     __syncthreads();
     if (wid == 0) {
       if (lane == 0) {
@@ -857,8 +914,8 @@ __global__ void __launch_bounds__(TEAM, 8) k_sweep_team(ModelCfg cfg, FrameSet<f
       __syncwarp();
       if (tc.nb > 0) advance_prefix(&c->frontier, fs.done + base, c->nrun, epoch, lane);
       if (go == 1 && !esc)
-        after_step(fs, c, c->attempt, base, r, li, *ws.orig, tc.act == ACT_BREAK_ADDED ? *ws.t : *ws.w,
-                   reinterpret_cast<const int*>(ws.scratch), lane);
+        after_step(fs, c, c->attempt, base, r, li, *v.orig, tc.act == ACT_BREAK_ADDED ? *v.t : *v.w,
+                   reinterpret_cast<const int*>(v.scratch), lane);
     }
   }
 }
@@ -1324,8 +1381,9 @@ __global__ void __launch_bounds__(32) k_tail(ModelCfg cfg, FrameSet<T> fs, int t
 
 // k_tail with a team (one CTA) per frame; warp 0 keeps the run list,
 // recentres and counts.
-template <int M>
-__global__ void __launch_bounds__(TEAM) k_tail_team(ModelCfg cfg, FrameSet<float> fs, int tail_peaks) {
+template <typename S>
+__global__ void __launch_bounds__(S::THREADS)
+    k_tail_team(const __grid_constant__ ModelCfg cfg, const __grid_constant__ FrameSet<typename S::T> fs, int tail_peaks) {
   extern __shared__ __align__(16) char smem[];
   __shared__ TeamCtl tc;
   __shared__ int s_nrun, s_more;
@@ -1333,14 +1391,12 @@ __global__ void __launch_bounds__(TEAM) k_tail_team(ModelCfg cfg, FrameSet<float
   const int f = blockIdx.x;
   FrameCtl* c = fs.ctl + f;
   if (!tail_ready(c, tail_peaks)) return;
-  WarpWS<float> ws = g32_team_ws(smem, cfg);
-  // warp 0's view for recentring (the trial tables' memory)
-  WarpWS<float> wr = ws;
+  typename S::WS ws = S::workspace(smem, cfg);
+  WarpWS<typename S::T> wr = S::aux(ws);
   {
-    unsigned short* roi = reinterpret_cast<unsigned short*>(smem + g32_team_bytes(cfg));
-    for (int i = tid; i < cfg.nroi; i += TEAM) roi[i] = fs.roi_xy[i];
-    ws.roi = roi;
-    wr.tab0 = ws.tab1;
+    unsigned short* roi = reinterpret_cast<unsigned short*>(smem + S::bytes(cfg));
+    for (int i = tid; i < cfg.nroi; i += S::THREADS) roi[i] = fs.roi_xy[i];
+    S::pixel_tables(cfg, fs, smem, ws, roi);
   }
   const int base = fs.pk_off[f];
   const long long fbase = (long long)f * fs.npix;
@@ -1355,13 +1411,12 @@ __global__ void __launch_bounds__(TEAM) k_tail_team(ModelCfg cfg, FrameSet<float
     long long loc = 0;   // lane i of warp 0: counter i of this sweep
     for (int r = 0; r < nrun; r++) {
       const int li = fs.run[base + r];
-      g32_prologue<M, TEAM_WARPS>(cfg, fs, fs.pk + base + li, ws, tid);
+      S::template prologue<S::THREADS>(cfg, fs, fs.pk + base + li, ws, tid);
       __syncthreads();
-      lm_step_g32<M>(cfg, fs, fbase, fs.pk + base + li, true, 0, ws, tc,
-                     fs.stepctr + (size_t)(base + li) * NCOUNTERS, tid);
+      S::step(cfg, fs, fbase, fs.pk + base + li, true, 0, ws, tc, fs.stepctr + (size_t)(base + li) * NCOUNTERS, tid);
       __threadfence();
       __syncthreads();
-      if (wid == 0 && lane < NCOUNTERS) loc += reinterpret_cast<const int*>(ws.scratch)[lane];
+      if (wid == 0 && lane < NCOUNTERS) loc += reinterpret_cast<const int*>(S::view(ws).scratch)[lane];
     }
     if (wid == 0) {
       const bool more = tail_end_sweep(cfg, fs, c, base, fbase, nrun, loc, wr, lane);

@@ -26,22 +26,40 @@ struct Kernels {
   void (*tail)(ModelCfg, FrameSet<T>, int) = k_tail<T, -1>;
   void (*team_sweep)(ModelCfg, FrameSet<T>) = nullptr;
   void (*team_tail)(ModelCfg, FrameSet<T>, int) = nullptr;
+  int team_threads = 0;
   size_t team_bytes = 0;
+
+  template <typename S>
+  void team(const ModelCfg& cfg) {
+    team_sweep = k_sweep_team<S>;
+    team_tail = k_tail_team<S>;
+    team_threads = S::THREADS;
+    team_bytes = S::bytes(cfg);
+  }
+  template <int M>
+  void g32(const ModelCfg& cfg) {
+    sweep = k_sweep<T, M>;
+    tail = k_tail<T, M>;
+    team<StepG32<M>>(cfg);
+  }
 };
 
 template <typename T>
 static Kernels<T> kernels(const ModelCfg& cfg) {
   Kernels<T> k;
   if constexpr (sizeof(T) == 4) {
-    if (gauss32<T>(cfg)) {
-      k.team_bytes = g32_team_bytes(cfg);
-      switch (cfg.model) {
-        case M_2DFIXED: k.sweep = k_sweep<T, M_2DFIXED>; k.tail = k_tail<T, M_2DFIXED>; k.team_sweep = k_sweep_team<M_2DFIXED>; k.team_tail = k_tail_team<M_2DFIXED>; break;
-        case M_2D: k.sweep = k_sweep<T, M_2D>; k.tail = k_tail<T, M_2D>; k.team_sweep = k_sweep_team<M_2D>; k.team_tail = k_tail_team<M_2D>; break;
-        case M_3D: k.sweep = k_sweep<T, M_3D>; k.tail = k_tail<T, M_3D>; k.team_sweep = k_sweep_team<M_3D>; k.team_tail = k_tail_team<M_3D>; break;
-        default: k.sweep = k_sweep<T, M_Z>; k.tail = k_tail<T, M_Z>; k.team_sweep = k_sweep_team<M_Z>; k.team_tail = k_tail_team<M_Z>; break;
-      }
+    switch (cfg.model) {
+      case M_2DFIXED: k.template g32<M_2DFIXED>(cfg); break;
+      case M_2D: k.template g32<M_2D>(cfg); break;
+      case M_3D: k.template g32<M_3D>(cfg); break;
+      case M_Z: k.template g32<M_Z>(cfg); break;
+      default: k.template team<StepTeam<float, 1>>(cfg); break;
     }
+  } else {
+    if (is_fft(cfg.model)) k.template team<StepTeam<double, 2>>(cfg);
+    else if (is_pupil(cfg.model)) k.template team<StepTeam<double, 3>>(cfg);
+    else if (is_spline(cfg.model)) k.template team<StepTeam<double, 1>>(cfg);
+    else k.template team<StepTeam<double, 0>>(cfg);
   }
   return k;
 }
@@ -103,7 +121,7 @@ cudaError_t Launch<T>::configure(const ModelCfg& cfg, Shapes* sh) {
   sh->team_smem = k.team_bytes + roi_table_bytes(cfg.nroi);
   if (k.team_sweep && raise_limit((const void*)k.team_sweep, sh->team_smem) == cudaSuccess &&
       raise_limit((const void*)k.team_tail, sh->team_smem) == cudaSuccess) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.team_sweep, TEAM, sh->team_smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.team_sweep, k.team_threads, sh->team_smem);
     if (e != cudaSuccess) return e;
     sh->team_grid = nsm * per_sm;
   }
@@ -121,7 +139,7 @@ template <typename T>
 cudaError_t Launch<T>::sweep(const ModelCfg& cfg, const FrameSet<T>& fs, const Shapes& sh, int grid, bool team,
                              cudaStream_t s) {
   const Kernels<T> k = kernels<T>(cfg);
-  if (team) k.team_sweep<<<grid, TEAM, sh.team_smem, s>>>(cfg, fs);
+  if (team) k.team_sweep<<<grid, k.team_threads, sh.team_smem, s>>>(cfg, fs);
   else k.sweep<<<grid, 32 * sh.warps, sh.smem, s>>>(cfg, fs);
   return cudaGetLastError();
 }
@@ -130,7 +148,7 @@ template <typename T>
 cudaError_t Launch<T>::tail(const ModelCfg& cfg, const FrameSet<T>& fs, const Shapes& sh, int tail_peaks,
                             cudaStream_t s) {
   const Kernels<T> k = kernels<T>(cfg);
-  if (sh.team_grid > 0) k.team_tail<<<fs.F, TEAM, sh.team_smem, s>>>(cfg, fs, tail_peaks);
+  if (sh.team_grid > 0) k.team_tail<<<fs.F, k.team_threads, sh.team_smem, s>>>(cfg, fs, tail_peaks);
   else k.tail<<<fs.F, 32, (sh.smem - roi_table_bytes(cfg.nroi)) / sh.warps + roi_table_bytes(cfg.nroi), s>>>(cfg, fs, tail_peaks);
   return cudaGetLastError();
 }
