@@ -426,14 +426,22 @@ struct Engine {
   }
 
   // Whether a sweep of this many RUNNING peaks (all frames) runs a peak per
-  // team.  A team steps a peak in about half a warp's time, but four warps
-  // together get less done than four warps on four peaks, so teams lose once
-  // the sweep has ready peaks for every warp: about one RUNNING peak in 16 is
-  // ready at a time in frames of 0.5 emitters / um^2 (64 frames of 512 x 512, a
-  // sweep of 214,000 peaks 4.6 ms against 4.2 ms, of 60,000 1.6 against 1.5, of
-  // 22,000 0.42 against 0.45; one frame of 3,355 0.63 against 1.03).
+  // team.  A team steps a peak in less than half a warp's time, but four warps
+  // on one peak get less done than four on four, so FP32 Gaussians want warps
+  // once there are ready peaks for every warp.  Ready, not RUNNING: the more
+  // footprints cover a pixel, the fewer.  At 3,040 warp slots teams and warps
+  // break even at 20,000 to 30,000 peaks of 2 footprints a pixel and at some
+  // 100,000 of 16 (sweeps, ms with teams / warps: 3d 53,000 peaks 1.64 / 1.86,
+  // 107,000 2.79 / 2.69, 215,000 4.6 / 4.2, all of 16 a pixel; Z, 2 a pixel,
+  // 8,000 peaks 0.08 / 0.15, 64,000 1.91 / 1.64).  The FP64 engine and the
+  // splines are worth a team at any load (fits, ms: 51,000 peaks in FP64
+  // 187 / 216, 51,000 spline peaks 303 / 689, 14,400 FFT PSF 346 / 818,
+  // 9,600 pupil function 375 / 1425).
   bool team_sweep(long long running) const {
-    return shapes.team_grid > 0 && running < 16LL * shapes.grid * shapes.warps;
+    if (shapes.team_grid == 0) return false;
+    if (prec == 64 || cfg.model >= M_SPLINE2D) return true;
+    const double cover = (double)running * cfg.nroi / ((double)F * npix);
+    return running < 6.0 * shapes.grid * shapes.warps * (1.0 + 0.3 * cover);
   }
 
   cudaError_t enqueue_sweep(bool team) {
