@@ -276,7 +276,7 @@ void mpSetWeights(saMPFit *mp_fit, double *w_bg, double *w_h, double *w_x, doubl
 void mpSetWeightsIndexing(saMPFit *mp_fit, double z_offset, double z_scale);
 /* No reference counterpart: how many non-overlapping groups of a frame step
  * at once in a sweep (1..8), or 0 (the default) to choose it from the
- * number of frames (8 for a lone frame, down to 2 as the frames fill the
+ * number of frames (16 for a few frames, down to 2 as the frames fill the
  * GPU).
  * The results do not depend on it.  Returns 0, or -1 on error. */
 int mpSetTeams(saMPFit *mp_fit, int teams);

@@ -2467,7 +2467,7 @@ void mpCleanup(saMPFit* mp) {
 }
 
 // ---- batched multi-plane fitting (no reference counterpart): many frames
-// per channel handle, one warp per frame.  The channels' frames are set with
+// per channel handle.  The channels' frames are set with
 // mpSetFrames, their images with saNewImages / saNewBackgrounds on each
 // fit_data[i]; the results are read per channel with saGetResultsBatch /
 // saGetPeakPropertyBatch.

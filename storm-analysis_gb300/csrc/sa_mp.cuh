@@ -6,10 +6,12 @@
 // A group is one peak per channel at the same index.  Its channels share
 // status and lambda; x / y are tied through the affine maps between the
 // planes, z (and, unless the heights are independent) the height through
-// z-dependent weighted averages of the channels' LM steps.  One warp runs a
-// frame's groups in index order, the reference's Gauss-Seidel order, so a
-// multi-frame batch is parallel over frames only.  The FP64 engine.
+// z-dependent weighted averages of the channels' LM steps.  A frame's groups
+// give the result of the reference's index order (Gauss-Seidel); the frames
+// of a batch are independent.  The FP64 engine.
 #pragma once
+
+#include <cooperative_groups.h>
 
 #include "sa_kernels.cuh"
 #include "sa_mp_types.h"
@@ -41,26 +43,50 @@ __device__ inline bool mp_error(const MPChan& c, long long fbase, const PeakRec&
   return __any_sync(0xffffffffu, fail);
 }
 
-// fn_calc_JH on the global state with the peak still added (the fi of the
-// preceding mFitCalcErr): gradient and packed upper Hessian into jh.
-__device__ inline SplinePos mp_jh(const MPChan& c, long long fbase, const PeakRec& w, WarpWS<double>& ws,
-                                  double* jh, int lane) {
+// The first look at a group's plane, in one pass over its ROI: mFitCalcErr
+// (multi_fit.c:111-195) and fn_calc_JH on the state with the peak still added
+// (gradient and packed upper Hessian into jh), the start shape on a roi x roi
+// grid (psfo: for the exclusions and the commit), and the base state without
+// the peak in the workspace (as mp_base_excl leaves it at the start anchor).
+// True (and no error) when some fi <= 0.  Three passes that each read the ROI
+// back from L2 and rebuilt fi from the fixed-point sums were a third of the
+// step; every sum keeps its order (a lane's pixels ascending, then the warp
+// sum).
+__device__ inline bool mp_start(const MPChan& c, long long fbase, const PeakRec& w, WarpWS<double>& ws,
+                                double* jh, double* psfo, double& dev, int lane) {
   const ModelCfg& cfg = c.cfg;
   const int k = cfg.jac;
+  for (int q = lane; q < cfg.roi * cfg.roi; q += 32) psfo[q] = 0.0;
+  __syncwarp();
   SplinePos s = shape_tables(cfg, w, ws, lane);
   double gxd, gyd;
   z_factors(cfg, cfg.model, w, gxd, gyd);
   double acc[32];
 #pragma unroll
   for (int i = 0; i < 32; i++) acc[i] = 0.0;
+  double d = 0.0;
+  bool fail = false;
   for (int p = lane; p < cfg.nroi; p += 32) {
     int rx, ry;
-    roi_rc(c.fs.roi_xy, p, rx, ry);
+    roi_rc(ws.roi, p, rx, ry);
     const long long kk = pix_index(cfg, w.xi, w.yi, rx, ry);
-    const double fi = fi_global(c.fs, fbase + kk);
+    Q2 Fq = acc_load<2>(c.fs.f, fbase + kk);
+    Q2 Bq = acc_load<2>(c.fs.bg, fbase + kk);
+    const int Cg = __ldcg(c.fs.cnt + fbase + kk);
     const double xv = __ldg(c.fs.x + fbase + kk);
-    const double rq = __ldg(c.fs.rqe + kk);
+    const double rq = __ldg(c.fs.rqe + kk), sc = __ldg(c.fs.scmos + kk);
+    const double fi = acc_value<2>(Fq) + acc_value<2>(Bq) / (double)Cg;   // fi_global
+    if (!(fi > 0.0)) fail = true;
+    else d += deviance(fi, xv);
     const double psf = psf_at(cfg, c.fs.aij, ws, s, rx, ry);
+    psfo[ry * cfg.roi + rx] = psf;
+    Fq = q_sub(Fq, quant_t<double>(contrib_f(w.p[PH], psf, rq)));
+    Bq = q_sub(Bq, quant_t<double>(contrib_bg(w.p[PBG], rq, sc)));
+    ws.Fb[p] = acc_value<2>(Fq);
+    ws.Bs[p] = acc_value<2>(Bq) + sc;
+    ws.R[p] = rq;
+    ws.X[p] = xv;
+    ws.IC[p] = ic_store<double>(Cg);
     const double t1 = 2.0 * (1.0 - xv / fi);
     const double t2 = 2.0 * xv / (fi * fi);
     double jt[MAX_JAC];
@@ -81,38 +107,9 @@ __device__ inline SplinePos mp_jh(const MPChan& c, long long fbase, const PeakRe
   }
   const double v = warp_transpose_sum32(acc, lane);
   if (lane < k + k * (k + 1) / 2) jh[lane] = v;
+  dev = warp_sum(d);
   __syncwarp();
-  return s;
-}
-
-// Subtract the peak (its shape tables current in ws) from the plane's image
-// and keep the base state of its ROI -- the fit image and background
-// without it, rqe, data, count with it -- in the workspace, as lm_step's
-// first loop does: the trials are then evaluated from the workspace.
-__device__ inline void mp_sub_base(const MPChan& c, long long fbase, const PeakRec& w, const SplinePos& s,
-                                   WarpWS<double>& ws, int lane) {
-  const ModelCfg& cfg = c.cfg;
-  for (int p = lane; p < cfg.nroi; p += 32) {
-    int rx, ry;
-    roi_rc(ws.roi, p, rx, ry);
-    const long long kk = pix_index(cfg, w.xi, w.yi, rx, ry);
-    const Q2 Fq = acc_load<2>(c.fs.f, fbase + kk);
-    const Q2 Bq = acc_load<2>(c.fs.bg, fbase + kk);
-    const int Cg = __ldcg(c.fs.cnt + fbase + kk);
-    const double rq = __ldg(c.fs.rqe + kk), sc = __ldg(c.fs.scmos + kk);
-    const double psf = psf_at(cfg, c.fs.aij, ws, s, rx, ry);
-    const Q2 cf = quant_t<double>(contrib_f(w.p[PH], psf, rq));
-    const Q2 cb = quant_t<double>(contrib_bg(w.p[PBG], rq, sc));
-    acc_red<2>(c.fs.f, fbase + kk, cf, -1);
-    acc_red<2>(c.fs.bg, fbase + kk, cb, -1);
-    atomicAdd(c.fs.cnt + fbase + kk, -1);
-    ws.Fb[p] = acc_value<2>(q_sub(Fq, cf));
-    ws.Bs[p] = acc_value<2>(q_sub(Bq, cb)) + sc;
-    ws.R[p] = rq;
-    ws.X[p] = __ldg(c.fs.x + fbase + kk);
-    ws.IC[p] = ic_store<double>(Cg);
-  }
-  __syncwarp();
+  return __any_sync(0xffffffffu, fail);
 }
 
 // The error of the trial w from the base state in ws (the peak added
@@ -137,22 +134,6 @@ __device__ inline bool mp_trial_error(const MPChan& c, const PeakRec& w, WarpWS<
   }
   dev = warp_sum(d);
   return __any_sync(0xffffffffu, fail);
-}
-
-// Add the accepted trial w (its shape in ws.psf) to the plane's image.
-__device__ inline void mp_add_from_ws(const MPChan& c, long long fbase, const PeakRec& w, WarpWS<double>& ws,
-                                      int lane) {
-  const ModelCfg& cfg = c.cfg;
-  for (int p = lane; p < cfg.nroi; p += 32) {
-    int rx, ry;
-    roi_rc(ws.roi, p, rx, ry);
-    const long long kk = pix_index(cfg, w.xi, w.yi, rx, ry);
-    const double rq = ws.R[p], sc = __ldg(c.fs.scmos + kk);
-    acc_red<2>(c.fs.f, fbase + kk, quant_t<double>(contrib_f(w.p[PH], ws.psf[p], rq)), +1);
-    acc_red<2>(c.fs.bg, fbase + kk, quant_t<double>(contrib_bg(w.p[PBG], rq, sc)), +1);
-    atomicAdd(c.fs.cnt + fbase + kk, 1);
-  }
-  __syncwarp();
 }
 
 // Add (+1) or subtract (-1) channel c's working peak (its shape computed here).
@@ -336,7 +317,7 @@ __device__ inline void mp_check_error(const MPChan* ch, const MPParams& p, int f
 // ---------------------------------------------------------------------------
 // The sweep, several groups at once.
 //
-// A frame's groups are taken in index order in batches of at most MP_TEAMS:
+// A frame's groups are taken in index order in batches of at most p.batch:
 // a batch is a run of consecutive RUNNING groups whose ROIs, grown by
 // MP_DIL pixels on every side, overlap in no plane.  Every group of a batch
 // takes its step at once, one team of warps (a warp per plane) each, on
@@ -406,7 +387,7 @@ __device__ inline int mp_team_step(const MPChan* ch, const MPParams& p, int f, i
     PeakRec r;
     load_rec(C.fs.pk + C.fs.pk_off[f] + g, r);
     double dev;
-    const bool fail = mp_error(C, fb, r, dev, lane);
+    const bool fail = mp_start(C, fb, r, wc, S.jh[c], psfo, dev, lane);
     if (lane == 0) S.orig[c] = r;   // the stored peak (mpResetWorkingPeaks restores it)
     if (!fail) r.error = dev;       // the return value is ignored (mp_fit.c:220)
     else if (lane == 0) K.ctr[c][C_NEGFI]++;
@@ -415,17 +396,7 @@ __device__ inline int mp_team_step(const MPChan* ch, const MPParams& p, int f, i
       r.added -= 1;
       S.w[c] = r;
     }
-    const SplinePos sp = mp_jh(C, fb, r, wc, S.jh[c], lane);
-    // the start shape on a roi x roi grid (for the exclusions and the commit)
-    for (int q = lane; q < C.cfg.roi * C.cfg.roi; q += 32) psfo[q] = 0.0;
     __syncwarp();
-    for (int q = lane; q < C.cfg.nroi; q += 32) {
-      int rx, ry;
-      roi_rc(wc.roi, q, rx, ry);
-      psfo[ry * C.cfg.roi + rx] = psf_at(C.cfg, C.fs.aij, wc, sp, rx, ry);
-    }
-    __syncwarp();
-    mp_base_excl(C, fb, r.xi, r.yi, r, psfo, wc, lane);
   }
   int cax = S.orig[c].xi, cay = S.orig[c].yi;
   const int x0 = S.orig[c].xi, y0 = S.orig[c].yi;
@@ -607,16 +578,37 @@ __device__ inline void mp_commit(const MPChan& C, int f, int g, const MPTeam& T,
   }
 }
 
-// mpIterateLM mp_fit.c:183-478 for frame blockIdx.x (batches of groups as
-// above; blockDim.x = 32 * nc * p.teams), then mFitRecenterPeaks per plane
-// and mpCheckError per group.
+// All CTAs of a frame (one, or a cluster): barrier with the image and record
+// writes before it visible behind it.
+__device__ __forceinline__ void frame_sync(int cl) {
+  if (cl == 1) __syncthreads();
+  else cooperative_groups::this_cluster().sync();
+}
+
+// mpIterateLM mp_fit.c:183-478 for one frame (batches of groups as above),
+// then mFitRecenterPeaks per plane and mpCheckError per group.
+//
+// A frame is a cluster of p.cl CTAs of p.teams teams each (blockDim.x =
+// 32 * nc * p.teams): a step is bound by the SM's FP64 pipes, so few frames are spread
+// over the SMs.
+// The CTAs share nothing but global memory and one word, the lowest escaped
+// group; each builds the same list of RUNNING groups (a window of p.window
+// groups at a time, their anchors in shared memory; a group's status and
+// anchors change by its own step only) and finds the same batches from it.
+// The list, the recentering test and the error test take a lane per group:
+// one thread reading record after record, with two barriers per group, took
+// longer than the steps once most groups had converged: a 256 x 256 frame of
+// 200 groups in two planes fitted in 71 ms so, in 54 with a lane per group
+// and one pass over the ROI at a step's start, and in 27 on 8 SMs; 64 such
+// frames in 128, 87 and 67 (on 4 SMs each).
 __global__ void __launch_bounds__(32 * MP_MAXCH * 2) k_mp_sweep(const MPChan* chans, MPParams p) {
   extern __shared__ __align__(16) char smem[];
-  const int nc = p.nc;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nc = p.nc, cl = p.cl, win = p.window, n_chunk = (win + 31) / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
   const int team = warp / nc, c = warp - team * nc;
   const int nthr = 32 * nc;
-  const int f = blockIdx.x;
+  const int f = blockIdx.x / cl, rank = blockIdx.x - f * cl;
+  const int gteam = team * cl + rank, n_teams = p.teams * cl;
   const size_t wstride = (size_t)p.ws_bytes + (((size_t)p.grid_doubles * 8 + 15) & ~(size_t)15);
   char* const ws_c = smem + (size_t)warp * wstride;
   double* const psfo = reinterpret_cast<double*>(ws_c + p.ws_bytes);
@@ -625,89 +617,104 @@ __global__ void __launch_bounds__(32 * MP_MAXCH * 2) k_mp_sweep(const MPChan* ch
   off += ((sizeof(MPTeam) * p.teams + 15) & ~(size_t)15);
   MPChan* ch = reinterpret_cast<MPChan*>(smem + off);
   off += ((sizeof(MPChan) * nc + 15) & ~(size_t)15);
-  int* bgrp = reinterpret_cast<int*>(smem + off);           // the batch's groups
-  int* bbox = bgrp + MP_TEAMS;                               // their grown ROIs per plane: x0, y0, x1, y1
-  int* sh = bbox + 4 * MP_TEAMS * MP_MAXCH;                  // nb, next, esc_min
+  int* grp = reinterpret_cast<int*>(smem + off);            // the window's RUNNING groups
+  int2* anc = reinterpret_cast<int2*>(grp + win);     // their anchors [plane][win]
+  int* cnt = reinterpret_cast<int*>(anc + nc * win);  // RUNNING groups per 32 of the window
+  int* escaped = cnt + n_chunk;                      // the lowest escaped group, two batches' turns
   for (int i = threadIdx.x; i < (int)(nc * sizeof(MPChan) / 4); i += blockDim.x)
     reinterpret_cast<int*>(ch)[i] = reinterpret_cast<const int*>(chans)[i];
   if (threadIdx.x < p.teams * MP_MAXCH) teams[threadIdx.x / MP_MAXCH].S.heights[threadIdx.x % MP_MAXCH] = 1.0;
-  __syncthreads();
+  if (threadIdx.x < 2) escaped[threadIdx.x] = INT_MAX;
+  frame_sync(cl);   // every CTA's words are set before another one writes them
   const MPChan& C = ch[c];
+  const long long fb = mp_fbase(C, f);
   WarpWS<double> wc = warp_ws<double>(ws_c, C.cfg, C.cfg.nroi);
   wc.roi = C.fs.roi_xy;
   const int nfit = ch[0].fs.nfit[f];
-  int base = 0;
-  while (base < nfit) {
-    if (threadIdx.x == 0) {
-      // the batch: consecutive RUNNING groups, grown ROIs disjoint in every plane
-      int nb = 0, g = base;
-      while (nb < p.teams && g < nfit) {
-        if (ch[0].fs.pk[ch[0].fs.pk_off[f] + g].status != RUNNING) {
-          g++;
-          continue;
-        }
-        bool clash = false;
-        int box[MP_MAXCH][4];
+  int turn = 0;
+  for (int base = 0; base < nfit; base += win) {
+    const int n_win = min(win, nfit - base);
+    const PeakRec* const q0 = ch[0].fs.pk + ch[0].fs.pk_off[f] + base;
+    for (int k = warp; k < n_chunk; k += n_warps) {
+      const int j = 32 * k + lane;
+      const unsigned m = __ballot_sync(0xffffffffu, j < n_win && __ldcg(&q0[j].status) == RUNNING);
+      if (lane == 0) cnt[k] = __popc(m);
+    }
+    __syncthreads();
+    int n_run = 0;
+    for (int k = 0; k < n_chunk; k++) n_run += cnt[k];
+    for (int k = warp; k < n_chunk; k += n_warps) {
+      const int j = 32 * k + lane;
+      const bool run = j < n_win && __ldcg(&q0[j].status) == RUNNING;
+      const unsigned m = __ballot_sync(0xffffffffu, run);
+      int at = __popc(m & ((1u << lane) - 1u));
+      for (int i = 0; i < k; i++) at += cnt[i];
+      if (run) {
+        grp[at] = base + j;
         for (int i = 0; i < nc; i++) {
-          const PeakRec* q = ch[i].fs.pk + ch[i].fs.pk_off[f] + g;
-          const int xi = q->xi, yi = q->yi, roi = ch[i].cfg.roi;
-          box[i][0] = xi - MP_DIL;
-          box[i][1] = yi - MP_DIL;
-          box[i][2] = xi + roi + MP_DIL;
-          box[i][3] = yi + roi + MP_DIL;
-          for (int m = 0; m < nb && !clash; m++) {
-            const int* o = bbox + 4 * (m * MP_MAXCH + i);
-            if (box[i][0] < o[2] && o[0] < box[i][2] && box[i][1] < o[3] && o[1] < box[i][3]) clash = true;
+          const PeakRec* q = ch[i].fs.pk + ch[i].fs.pk_off[f] + base + j;
+          anc[i * win + at] = make_int2(__ldcg(&q->xi), __ldcg(&q->yi));
+        }
+      }
+    }
+    __syncthreads();
+    for (int pos = 0; pos < n_run;) {
+      // the batch: the next groups of the list whose grown ROIs are disjoint
+      // in every plane (lane m: group m of the batch)
+      int nb = 1;
+      for (; nb < p.batch && pos + nb < n_run; nb++) {
+        bool clash = false;
+        if (lane < nb) {
+          for (int i = 0; i < nc; i++) {
+            const int2 a = anc[i * win + pos + lane], b = anc[i * win + pos + nb];
+            const int reach = ch[i].cfg.roi + 2 * MP_DIL;
+            clash |= abs(a.x - b.x) < reach && abs(a.y - b.y) < reach;
           }
         }
-        if (clash) break;
-        for (int i = 0; i < nc; i++)
-          for (int k = 0; k < 4; k++) bbox[4 * (nb * MP_MAXCH + i) + k] = box[i][k];
-        bgrp[nb++] = g++;
+        if (__any_sync(0xffffffffu, clash)) break;
       }
-      sh[0] = nb;
-      sh[1] = g;
-      sh[2] = INT_MAX;
-    }
-    __syncthreads();
-    const int nb = sh[0];
-    if (nb == 0) {
-      base = sh[1];
-      __syncthreads();
-      continue;
-    }
-    // a lone group's step cannot meet another's: unbounded (no escape)
-    int esc = 0;
-    if (team < nb) {
-      esc = mp_team_step(ch, p, f, bgrp[team], teams[team], wc, psfo, c, lane, team, nthr, nb > 1);
-      if (esc && c == 0 && lane == 0) atomicMin(&sh[2], team);
-    }
-    __syncthreads();
-    const int emin = sh[2];
-    if (team < nb && team < emin) mp_commit(C, f, bgrp[team], teams[team], wc, psfo, c, lane);
-    __syncthreads();
-    if (emin < nb) {
-      // the escaped group alone, on the committed state
-      if (team == 0) {
-        mp_team_step(ch, p, f, bgrp[emin], teams[0], wc, psfo, c, lane, 0, nthr, false);
-        mp_commit(C, f, bgrp[emin], teams[0], wc, psfo, c, lane);
+      // a lone group's step cannot meet another's: unbounded (no escape)
+      if (gteam < nb) {
+        const int esc = mp_team_step(ch, p, f, grp[pos + gteam], teams[team], wc, psfo, c, lane, team, nthr, nb > 1);
+        if (esc && c == 0 && lane == 0) {
+          for (int r = 0; r < cl; r++)
+            atomicMin(cl == 1 ? escaped + turn : cooperative_groups::this_cluster().map_shared_rank(escaped + turn, r),
+                      gteam);
+        }
       }
-      base = bgrp[emin] + 1;
-    } else {
-      base = sh[1];
+      frame_sync(cl);
+      const int emin = escaped[turn];
+      turn ^= 1;
+      if (threadIdx.x == 0) escaped[turn] = INT_MAX;
+      if (gteam < nb && gteam < emin) mp_commit(C, f, grp[pos + gteam], teams[team], wc, psfo, c, lane);
+      frame_sync(cl);
+      if (emin < nb) {
+        // the escaped group alone, on the committed state
+        if (gteam == 0) {
+          mp_team_step(ch, p, f, grp[pos + emin], teams[0], wc, psfo, c, lane, 0, nthr, false);
+          mp_commit(C, f, grp[pos + emin], teams[0], wc, psfo, c, lane);
+        }
+        pos += emin + 1;
+        frame_sync(cl);
+      } else {
+        pos += nb;
+      }
     }
-    __syncthreads();
   }
-  // mFitRecenterPeaks multi_fit.c:1644-1690: team 0, a warp per plane
-  if (team == 0) {
-    const long long fb = mp_fbase(C, f);
-    for (int g = 0; g < nfit; g++) {
-      PeakRec* q = C.fs.pk + C.fs.pk_off[f] + g;
+  // mFitRecenterPeaks multi_fit.c:1644-1690: a warp per plane of every team,
+  // 32 groups at a time (the image's sums are whole numbers: any order)
+  for (int base = 32 * gteam; base < nfit; base += 32 * n_teams) {
+    PeakRec* const q0 = C.fs.pk + C.fs.pk_off[f] + base;
+    bool moved = false;
+    if (base + lane < nfit && __ldcg(&q0[lane].status) == RUNNING) {
+      const double dx = __ldcg(&q0[lane].p[PX]) - __ldcg(&q0[lane].xi);
+      const double dy = __ldcg(&q0[lane].p[PY]) - __ldcg(&q0[lane].yi);
+      moved = (dx < -0.25) || (dx > 1.25) || (dy < -0.25) || (dy > 1.25);
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, moved); todo; todo &= todo - 1) {
+      PeakRec* q = q0 + (__ffs(todo) - 1);
       PeakRec r;
       load_rec(q, r);
-      if (r.status != RUNNING) continue;
-      const double dx = r.p[PX] - r.xi, dy = r.p[PY] - r.yi;
-      if (!((dx < -0.25) || (dx > 1.25) || (dy < -0.25) || (dy > 1.25))) continue;
       mp_add(C, fb, r, wc, -1, lane);
       r.added -= 1;
       r.xi = (int)floor(r.p[PX]);
@@ -715,8 +722,9 @@ __global__ void __launch_bounds__(32 * MP_MAXCH * 2) k_mp_sweep(const MPChan* ch
       const int chk = base_check(C.cfg, r);
       if (chk) {
         if (lane == 0) {
-          C.fs.ctl[f].ctr[C_LOST]++;
-          C.fs.ctl[f].ctr[chk == 1 ? C_MARGIN : C_NEGH]++;
+          unsigned long long* ctr = reinterpret_cast<unsigned long long*>(C.fs.ctl[f].ctr);
+          atomicAdd(ctr + C_LOST, 1ull);
+          atomicAdd(ctr + (chk == 1 ? C_MARGIN : C_NEGH), 1ull);
         }
         r.status = ERROR;
       } else {
@@ -728,32 +736,32 @@ __global__ void __launch_bounds__(32 * MP_MAXCH * 2) k_mp_sweep(const MPChan* ch
       __syncwarp();
     }
   }
-  __syncthreads();
-  // mpCheckError mp_fit.c:43-68 for every group: team 0, a warp per plane
-  for (int g = 0; g < nfit; g++) {
-    if (threadIdx.x == 0) {
-      bool bad = false;
-      for (int i = 0; i < nc; i++) bad |= (ch[i].fs.pk[ch[i].fs.pk_off[f] + g].status == ERROR);
-      sh[0] = bad;
-    }
-    __syncthreads();
-    if (sh[0] && team == 0) {
-      PeakRec* q = C.fs.pk + C.fs.pk_off[f] + g;
+  frame_sync(cl);
+  // mpCheckError mp_fit.c:43-68: a plane's peak goes where another plane's is
+  // in ERROR (each warp writes its own plane's records only, and a record
+  // made ERROR here belongs to a group that has one already)
+  for (int base = 32 * gteam; base < nfit; base += 32 * n_teams) {
+    PeakRec* const q0 = C.fs.pk + C.fs.pk_off[f] + base;
+    bool bad = false;
+    if (base + lane < nfit && __ldcg(&q0[lane].status) != ERROR)
+      for (int i = 0; i < nc; i++) bad |= __ldcg(&ch[i].fs.pk[ch[i].fs.pk_off[f] + base + lane].status) == ERROR;
+    for (unsigned todo = __ballot_sync(0xffffffffu, bad); todo; todo &= todo - 1) {
+      PeakRec* q = q0 + (__ffs(todo) - 1);
       PeakRec r;
       load_rec(q, r);
-      if (r.status != ERROR) {
-        mp_add(C, mp_fbase(C, f), r, wc, -1, lane);
-        r.added -= 1;
-      }
+      mp_add(C, fb, r, wc, -1, lane);
+      r.added -= 1;
       r.status = ERROR;
       __syncwarp();
       if (lane == 0) *q = r;
+      __syncwarp();
     }
-    __syncthreads();
   }
-  if (p.unconv && warp == 0) {
+  frame_sync(cl);
+  if (p.unconv && rank == 0 && warp == 0) {
+    const PeakRec* q0 = ch[0].fs.pk + ch[0].fs.pk_off[f];
     int n = 0;
-    for (int g = lane; g < nfit; g += 32) n += (ch[0].fs.pk[ch[0].fs.pk_off[f] + g].status == RUNNING);
+    for (int g = lane; g < nfit; g += 32) n += (__ldcg(&q0[g].status) == RUNNING);
     n = warp_sum_int(n);
     if (lane == 0) p.unconv[f] = n;
   }

@@ -7,7 +7,9 @@
 namespace sa {
 
 constexpr int MP_MAXCH = 8;
-constexpr int MP_TEAMS = 8;   // groups of a frame stepping at once (a batch) at most
+constexpr int MP_TEAMS = 8;     // groups of a frame stepping at once (a batch) at most
+constexpr int MP_BATCH = 16;    // the same where they spread over 8 SMs (at most 32: a lane each)
+constexpr int MP_WINDOW = 256; // groups listed at a time (fewer where shared memory is short)
 enum { MP_ARB = 0, MP_DAO = 1 };
 
 // One channel: its engine's model and frame set.
@@ -25,7 +27,10 @@ struct MPParams {
   int start, stop;   // k_mp_newpeaks: the new groups (stop < 0: to the frame's last)
   int fix_heights;   // k_mp_newpeaks: give the new groups their channels' mean height
   int* unconv;       // k_mp_sweep: RUNNING groups per frame after the sweep (may be null)
-  int teams;         // k_mp_sweep: groups of a frame stepped at once (1 .. 8)
+  int teams;         // k_mp_sweep: teams of a CTA
+  int cl;            // k_mp_sweep: CTAs of a frame (a cluster)
+  int batch;         // k_mp_sweep: groups of a frame stepped at once (at most teams * cl)
+  int window;        // k_mp_sweep: groups listed at a time
   int grid_doubles;  // k_mp_sweep: a plane's roi x roi shape grid (the largest of the planes')
 };
 

@@ -296,3 +296,34 @@ def test_mp_batch_equals_single_frames(teams):
             for k in ("x", "y", "height", "background", "xsigma", "status", "iterations"):
                 assert numpy.array_equal(out[c][k][o:o + n], single[fr][c][k]), (c, fr, k)
             o += n
+
+
+@pytest.mark.parametrize("frames,groups", [(1, 300), (2, 256), (20, 33), (115, 31), (153, 5)])
+def test_mp_frames_over_several_sms(frames, groups):
+    """However many SMs a frame is given (8, 8, 4, 2, 1 for these frame
+    counts) and whether its groups fit one window of the sweep's list (256)
+    or not, every frame's results are bit for bit those of one group after
+    another (mpSetTeams 1)."""
+    from sa_gb300 import mp_fit_dao_c, synth
+    side = 224 if groups > 100 else 96
+    wls = [synth.multiplane_workload(nx=side, ny=side + 8, n_emitters=groups, seed=s) for s in (51, 52)]
+    nc, shape = wls[0]["n_channels"], (wls[0]["ny"], wls[0]["nx"])
+    outs = []
+    for teams, n in ((1, min(frames, 2)), (0, frames)):
+        f = mp_fit_dao_c.MPFitDao2D(n_channels=nc, roi_size=10, sigma_range=(1.0, 3.0))
+        for c in range(nc):
+            f.initializeChannel(numpy.ones(shape), numpy.zeros(shape), c)
+        f.setMapping(*wls[0]["maps"])
+        f.setWeights(verbose=False)
+        assert f.clib.mpSetTeams(f.mfit, teams) == 0
+        use = [wls[k % 2] for k in range(n)]
+        images = [numpy.stack([wl["images"][c] for wl in use]) for c in range(nc)]
+        bgs = [numpy.stack([wl["backgrounds"][c] for wl in use]) for c in range(nc)]
+        outs.append(f.fitBatch(images, bgs, [wl["peaks"] for wl in use], "finder", max_iterations=100)[0])
+        f.cleanup(verbose=False)
+    for c in range(nc):
+        for k in ("x", "y", "height", "background", "xsigma", "error", "status", "iterations"):
+            if k not in outs[0][c]:
+                continue
+            one, all_ = numpy.asarray(outs[0][c][k]), numpy.asarray(outs[1][c][k])
+            assert numpy.array_equal(all_, numpy.resize(one, all_.size)), (c, k)
