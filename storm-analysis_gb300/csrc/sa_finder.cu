@@ -49,8 +49,14 @@ void ferr(const char* fmt, ...) {
 constexpr int kThreads = 256;
 constexpr int kSlowTR = 64;   // output rows per block of the slow-axis pass
 constexpr int kTC = 32;       // columns per block of the slow-axis and 2D passes
+constexpr int kFastThreads = 128;   // threads per block of the float-pair fast-axis pass at most
+constexpr int kFastQ = 4;     // neighbouring outputs of one of its threads
+constexpr int kSlowQ = 4;     // rows of a thread of the float-pair slow-axis pass
+constexpr int kFastRows = 8;  // rows of one of its blocks at most
 constexpr int k2dTR = 16;     // output rows per block of the 2D pass
 constexpr size_t kSmemMax = 200 * 1024;
+constexpr size_t kSlowSmemMax = 208 * 1024;   // float-pair slow-axis pass: its taps are held twice
+constexpr size_t kFastSmem = 36 * 1024;   // of the rows of a fast-axis block: six blocks fit an SM
 
 template <typename P>
 void dfree(P*& p) {
@@ -157,9 +163,29 @@ k_conv_slow(const double* __restrict__ in, double* __restrict__ out, int R, int 
 // 2^-48 of the running sum is lost: the result agrees with the FP64 sum to
 // ~1e-14 of its magnitude.  The explicit-rounding intrinsics keep the
 // compiler from fusing the two-sum steps.
+//
+// The FP64 pipe (an instruction of a warp takes a scheduler 64 cycles) is
+// kept off the path as far as the formats allow: an input is split with
+// integer operations (nearest float and remainder; values outside the floats'
+// normal range take the FP64 conversions), the first pass hands its pairs to
+// the second as they are, and only the last sum becomes a double.
 __device__ __forceinline__ float2 ff_split(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+  if (e - 963u < 186u) {   // 2^-60 <= |v| < 2^126: both floats are normal or zero
+    const unsigned long long r = b + 0x10000000ull;         // the upper 23 bits, rounded (half up)
+    const unsigned hi = (unsigned)(r >> 32) & 0x7fffffffu;
+    const float h = __uint_as_float(((hi - (896u << 20)) << 3) | ((unsigned)r >> 29) | ((unsigned)(b >> 32) & 0x80000000u));
+    const int rem = (int)((unsigned)r & 0x1fffffffu) - 0x10000000;          // v - h in units of 2^(e - 1075)
+    const float unit = __uint_as_float(((e - 948u) << 23) | ((unsigned)(b >> 32) & 0x80000000u));
+    return make_float2(h, __int2float_rn(rem) * unit);
+  }
   const float h = __double2float_rn(v);
   return make_float2(h, __double2float_rn(v - (double)h));
+}
+
+__host__ __device__ __forceinline__ int fast_units(int C, bool two) {
+  return two ? (C + 2 * kFastQ - 1) / (2 * kFastQ) : (C + kFastQ - 1) / kFastQ;
 }
 
 __device__ __forceinline__ void ff_tap(float2 w, float2 x, float& sh, float& sl) {
@@ -175,56 +201,202 @@ __device__ __forceinline__ void ff_tap(float2 w, float2 x, float& sh, float& sl)
   sl = __fsub_rn(t, __fsub_rn(sh, s));
 }
 
-__global__ void __launch_bounds__(kThreads)
-k_conv_fast_ff(const double* __restrict__ in, double* __restrict__ out, int R, int C,
-               const float2* __restrict__ w, int b0, int nb, const int* __restrict__ flag) {
-  extern __shared__ float2 smf[];
-  const int r = blockIdx.x, f = blockIdx.y;
-  if (!flag[f]) return;
-  float2* ws = smf;
-  float2* ext = smf + nb;
-  const size_t row = ((size_t)f * R + r) * C;
-  for (int j = threadIdx.x; j < nb; j += blockDim.x) ws[j] = w[j];
-  int base = (-b0 - nb + 1) % C;
-  if (base < 0) base += C;
-  const int next = C + nb - 1;
-  for (int t = threadIdx.x; t < next; t += blockDim.x) ext[t] = ff_split(in[row + (t + base) % C]);
-  __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    const float2* e = ext + c + nb - 1;
-    float sh = 0.0f, sl = 0.0f;
-    for (int j = 0; j < nb; ++j) ff_tap(ws[j], e[-j], sh, sl);
-    out[row + c] = (double)sh + (double)sl;
+// Two sums side by side in the packed FP32 instructions (two additions or
+// multiply-adds an instruction, each rounded as the scalar one): the same
+// steps, the same bits.  A pair of values is (high, high, low, low).
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+// a - b: the product with -1 is exact
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, f2(-1.0f, -1.0f), a); }
+
+struct FF1 {   // one value or sum: a float pair
+  float2 v;
+};
+struct FF2 {   // two of them
+  F2 h, l;
+};
+__device__ __forceinline__ void ff_zero(FF1& s) { s.v = make_float2(0.0f, 0.0f); }
+__device__ __forceinline__ void ff_zero(FF2& s) { s.h = s.l = f2(0.0f, 0.0f); }
+__device__ __forceinline__ void ff_add_tap(FF1 w, FF1 x, FF1& s) { ff_tap(w.v, x.v, s.v.x, s.v.y); }
+// (w.l holds the low parts negated, so that the negated rounding error needs
+// no negations of its own)
+__device__ __forceinline__ void ff_add_tap(FF2 w, FF2 x, FF2& a) {
+  const F2 nh = f2_mul(w.h, f2(-1.0f, -1.0f));   // once a tap: the same for all outputs
+  const F2 p = f2_mul(w.h, x.h);
+  F2 e = f2_fma(nh, x.h, p);
+  e = f2_fma(nh, x.l, e);
+  e = f2_fma(w.l, x.h, e);
+  const F2 s = f2_add(a.h, p);
+  const F2 v = f2_sub(s, a.h);
+  F2 t = f2_add(f2_sub(a.h, f2_sub(s, v)), f2_sub(p, v));
+  t = f2_sub(f2_add(t, a.l), e);
+  a.h = f2_add(s, t);
+  a.l = f2_sub(t, f2_sub(a.h, s));
+}
+__device__ __forceinline__ FF1 ff_weight(float2 w, FF1) { return FF1{w}; }
+__device__ __forceinline__ FF2 ff_weight(float2 w, FF2) { return FF2{f2(w.x, w.x), f2(-w.y, -w.y)}; }
+
+// NQ sums (or pairs of sums) of na taps each, over neighbouring outputs:
+// output q takes tap i from x(na - 1 - i + q).  A value is read once and
+// serves NQ outputs from a ring of registers, as a tap does: one output at a
+// time read two words from shared memory for each tap and waited for one
+// chain of additions.  Each sum keeps the order of its taps.  What bounds it is
+// the FP32 pipe, 15 operations a tap: 32 frames of 534 x 534 and 81 taps take
+// it 300 us, the slow-axis pass 370 and the fast-axis pass (which also splits
+// the doubles and keeps the image) 410; 490 and 440 + 26 before.
+template <int NQ, typename V, typename X>
+__device__ __forceinline__ void ff_sums(const V* ws, int na, X x, V* sum) {
+  V ring[NQ];   // ring[(q - i) mod NQ] = x(na - 1 - i + q)
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    ff_zero(sum[q]);
+    if (q) ring[q] = x(na - 1 + q);
+  }
+  for (int i0 = 0; i0 < na; i0 += NQ) {
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+      if (i0 + u >= na) break;
+      ring[(NQ - u) % NQ] = x(na - 1 - i0 - u);
+      const V w = ws[i0 + u];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) ff_add_tap(w, ring[(q - u + NQ) % NQ], sum[q]);
+    }
   }
 }
 
+__device__ __forceinline__ void ff_store(FF1 v, float2* o, int c, int, int C) {
+  if (c < C) o[c] = v.v;
+}
+__device__ __forceinline__ void ff_store(FF2 v, float2* o, int c, int half, int C) {
+  const float2 h = f2_get(v.h), l = f2_get(v.l);
+  if (c < min(half, C)) o[c] = make_float2(h.x, l.x);
+  if (c < half && c + half < C) o[c + half] = make_float2(h.y, l.y);
+}
+
+// kFastQ outputs (FF2: two times kFastQ, half a row apart) a thread, rb rows
+// a block.  Staged values are spread by one in four (spread 2) so that the
+// threads of a warp, kFastQ values apart, meet no bank twice; rows that fill
+// the shared memory are not (spread 31).  old (memo): the rows read are kept
+// there for the next call's comparison (matched_filter.c:135-139).
+__host__ __device__ __forceinline__ int fast_at(int t, int spread) { return t + (t >> spread); }
+
+template <typename V>
+__global__ void __launch_bounds__(kFastThreads, 6)
+k_conv_fast_ff(const double* __restrict__ in, float2* __restrict__ out, int R, int C,
+               const float2* __restrict__ w, int b0, int nb, const int* __restrict__ flag, int rb, int spread,
+               double* __restrict__ old) {
+  extern __shared__ __align__(16) char smc[];
+  const int f = blockIdx.y, r0 = blockIdx.x * rb;
+  if (!flag[f]) return;
+  constexpr bool two = sizeof(V) == sizeof(FF2);
+  const int rows = min(rb, R - r0);
+  const int nu = fast_units(C, two);                 // threads' units of a row
+  const int half = two ? nu * kFastQ : C;
+  const int next = nu * kFastQ + nb - 1, pitch = fast_at(next, spread) + 1;
+  V* ws = reinterpret_cast<V*>(smc);
+  V* ext = ws + nb;
+  const size_t row0 = ((size_t)f * R + r0) * C;
+  for (int j = threadIdx.x; j < nb; j += blockDim.x) ws[j] = ff_weight(w[j], V());
+  int base = (-b0 - nb + 1) % C;
+  if (base < 0) base += C;
+  const auto wrap = [&](int i) {   // once round at most, but for rows shorter than the taps
+    while (i >= C) i -= C;
+    return i;
+  };
+  for (int r = 0; r < rows; ++r) {
+    const double* src = in + row0 + (size_t)r * C;
+    double* keep = old + row0 + (size_t)r * C;
+#pragma unroll 2
+    for (int t = threadIdx.x; t < next; t += blockDim.x) {
+      const int i = wrap(t + base);
+      const double va = src[i];
+      const float2 a = ff_split(va);
+      if (old && t < half) keep[i] = va;
+      if constexpr (two) {
+        const int i2 = wrap(t + half + base);
+        const double vb = src[i2];
+        const float2 b = ff_split(vb);
+        if (old && t < half && t + half < C) keep[i2] = vb;
+        ext[r * pitch + fast_at(t, spread)] = FF2{f2(a.x, b.x), f2(a.y, b.y)};
+      } else {
+        ext[r * pitch + fast_at(t, spread)] = FF1{a};
+      }
+    }
+  }
+  __syncthreads();
+  for (int u = threadIdx.x; u < rows * nu; u += blockDim.x) {
+    const int r = u / nu, c = (u - r * nu) * kFastQ;
+    const V* e = ext + r * pitch;
+    V sum[kFastQ];
+    ff_sums<kFastQ>(ws, nb, [&](int t) { return e[fast_at(c + t, spread)]; }, sum);
+#pragma unroll
+    for (int q = 0; q < kFastQ; ++q) ff_store(sum[q], out + row0 + (size_t)r * C, c + q, half, C);
+  }
+}
+
+// Slow axis: two columns and kSlowQ rows a thread; a block of 256 threads
+// covers 32 columns x kSlowTR rows, one of 64 threads a quarter of the rows.
 __global__ void __launch_bounds__(kThreads)
-k_conv_slow_ff(const double* __restrict__ in, double* __restrict__ out, int R, int C,
+k_conv_slow_ff(const float2* __restrict__ in, double* __restrict__ out, int R, int C,
                const float2* __restrict__ w, int a0, int na, const int* __restrict__ flag) {
-  extern __shared__ float2 smf[];
+  extern __shared__ __align__(16) char smc[];
   const int f = blockIdx.z;
   if (!flag[f]) return;
-  const int c0 = blockIdx.x * kTC, r0 = blockIdx.y * kSlowTR;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTC + tx;
-  float2* ws = smf;
-  float2* ext = smf + na;
+  constexpr int W2 = kTC / 2;
+  const int ny = blockDim.y, TR = kSlowQ * ny;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int c = blockIdx.x * kTC + 2 * tx, r0 = blockIdx.y * TR;
+  FF2* ws = reinterpret_cast<FF2*>(smc);
+  FF2* ext = ws + na;
   const size_t fb = (size_t)f * R * C;
-  for (int j = tid; j < na; j += kThreads) ws[j] = w[j];
+  for (int j = ty * W2 + tx; j < na; j += W2 * ny) ws[j] = ff_weight(w[j], FF2());
   int base = (r0 - a0 - na + 1) % R;
   if (base < 0) base += R;
-  const int nrows = kSlowTR + na - 1;
-  const int c = c0 + tx;
-  for (int t = ty; t < nrows; t += kThreads / kTC)
-    ext[t * kTC + tx] = (c < C) ? ff_split(in[fb + (size_t)((base + t) % R) * C + c]) : make_float2(0.0f, 0.0f);
+  const int nrows = TR + na - 1;
+  for (int t = ty; t < nrows; t += ny) {
+    const float2* p = in + fb + (size_t)((base + t) % R) * C + c;
+    const float2 z = make_float2(0.0f, 0.0f);
+    const float2 a = c < C ? p[0] : z, b = c + 1 < C ? p[1] : z;
+    ext[t * W2 + tx] = FF2{f2(a.x, b.x), f2(a.y, b.y)};
+  }
   __syncthreads();
-  if (c >= C) return;
-  for (int q = ty; q < kSlowTR; q += kThreads / kTC) {
-    const int r = r0 + q;
-    if (r >= R) break;
-    const float2* e = ext + (q + na - 1) * kTC + tx;
-    float sh = 0.0f, sl = 0.0f;
-    for (int i = 0; i < na; ++i) ff_tap(ws[i], e[-i * kTC], sh, sl);
-    out[fb + (size_t)r * C + c] = (double)sh + (double)sl;
+  const int q0 = ty * kSlowQ;
+  if (c >= C || r0 + q0 >= R) return;
+  FF2 sum[kSlowQ];
+  ff_sums<kSlowQ>(ws, na, [&](int t) { return ext[(q0 + t) * W2 + tx]; }, sum);
+#pragma unroll
+  for (int q = 0; q < kSlowQ; ++q) {
+    if (r0 + q0 + q >= R) break;
+    const float2 h = f2_get(sum[q].h), l = f2_get(sum[q].l);
+    double* o = out + fb + (size_t)(r0 + q0 + q) * C + c;
+    o[0] = (double)h.x + (double)l.x;
+    if (c + 1 < C) o[1] = (double)h.y + (double)l.y;
   }
 }
 
@@ -284,67 +456,84 @@ struct LMax {
 // conversions of the reference (y: truncation of yi -/+ radius; x: ceil
 // radius; radius**2 truncated to int).  Ties go to the pixel with the larger
 // row and column.
-__device__ bool is_local_max(const LMax& a, const double* fimg, int zi, int yi, int xi, double cur) {
-  const int sz = max(zi - a.z_range, 0), ez = min(zi + a.z_range, a.Z - 1);
-  const int sy = max((int)(yi - a.radius), 0), ey = min((int)(yi + a.radius), a.R - 1);
-  const int sx = max(xi - a.cr, 0), ex = min(xi + a.cr, a.C - 1);
-  // A necessary condition first: the 3 x 3 neighbourhood in the candidate's
-  // own plane (part of the search below).  Most candidates sit on the slope
-  // of a peak and fail here after a few reads; the outcome is the same
-  // since the test is a conjunction over the search region.
-  {
-    const double* p = fimg + (size_t)zi * a.R * a.C;
-    for (int y = max(yi - 1, sy); y <= min(yi + 1, ey); ++y)
-      for (int x = max(xi - 1, sx); x <= min(xi + 1, ex); ++x) {
-        if ((x - xi) * (x - xi) + (y - yi) * (y - yi) > a.rr) continue;
-        const double v = p[(size_t)y * a.C + x];
-        if (y <= yi && x <= xi) {
-          if (v > cur) return false;
-        } else if (v >= cur) {
-          return false;
-        }
-      }
+// The search is comparisons only.  Above a threshold of 0 or more they are
+// made on the doubles' bit patterns (kBits): in order for positive numbers,
+// negative ones come out below, a NaN passes no comparison as before -- the
+// FP64 pipe takes 64 cycles for what the integer units do in four.
+template <bool kBits>
+__device__ __forceinline__ bool above(double v, double cur, bool or_equal) {
+  if (kBits) {
+    const long long b = __double_as_longlong(v), c = __double_as_longlong(cur);
+    return (or_equal ? b >= c : b > c) && b <= 0x7ff0000000000000ll;
   }
-  for (int z = sz; z <= ez; ++z) {
-    const double* p = fimg + (size_t)z * a.R * a.C;
-    for (int y = sy; y <= ey; ++y) {
-      const int dy = (y - yi) * (y - yi);
-      const double* row = p + (size_t)y * a.C;
-      for (int x = sx; x <= ex; ++x) {
-        const int dx = (x - xi) * (x - xi);
-        if (dx + dy > a.rr) continue;
-        const double v = row[x];
-        if (y <= yi && x <= xi) {
-          if (v > cur) return false;
-        } else if (v >= cur) {
-          return false;
-        }
-      }
+  return or_equal ? v >= cur : v > cur;
+}
+
+// Is the candidate at (zi, yi, xi) below or level with a neighbour next to it
+// in its own plane (part of the search below)?  Most candidates sit on the
+// slope of a peak and fail here; the outcome is the same since the test is a
+// conjunction over the search region.
+template <bool kBits>
+__device__ __forceinline__ bool beaten_nearby(const LMax& a, const double* p, int sy, int ey, int yi, int xi,
+                                              double cur) {
+  bool beaten = false;
+#pragma unroll
+  for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+    for (int dx = -1; dx <= 1; ++dx) {
+      const int y = yi + dy, x = xi + dx;
+      if ((dx == 0 && dy == 0) || y < sy || y > ey || x < 0 || x >= a.C || abs(dx) > a.cr || dx * dx + dy * dy > a.rr)
+        continue;
+      beaten |= above<kBits>(p[(size_t)y * a.C + x], cur, !(dy <= 0 && dx <= 0));
     }
-  }
-  return true;
+  return beaten;
 }
 
 // One warp per (frame, plane, row): candidate bits by ballot, row count.
+// What passes the look at its neighbours is searched by the whole warp, a
+// lane per pixel of the search box: a lane of its own waited for one load
+// after another (32 frames of 534 x 534: 370 us so, 127 now).
+// kBits: threshold >= 0.
+template <bool kBits>
 __global__ void k_lmax_mark(LMax a) {
   const int warp = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (warp >= a.nrows) return;
   const int y = warp % a.R, fz = warp / a.R, zi = fz % a.Z, f = fz / a.Z;
   const double* fimg = a.img + (size_t)f * a.Z * a.R * a.C;
-  const double* row = fimg + ((size_t)zi * a.R + y) * a.C;
+  const double* plane = fimg + (size_t)zi * a.R * a.C;
+  const double* row = plane + (size_t)y * a.C;
   const int32_t* tk = a.taken + (size_t)warp * a.C;
   uint32_t* bits = a.bits + (size_t)warp * a.W;
   const bool row_in = y >= a.margin && y < a.R - a.margin;
+  const int sz = max(zi - a.z_range, 0), ez = min(zi + a.z_range, a.Z - 1);
+  const int sy = max((int)(y - a.radius), 0), ey = min((int)(y + a.radius), a.R - 1);
   int cnt = 0;
   for (int w = 0; w < a.W; ++w) {
     const int x = w * 32 + lane;
     bool flag = false;
+    double cur = 0.0;
     if (row_in && x >= a.margin && x < a.C - a.margin) {
-      const double cur = row[x];
-      if (cur > a.threshold && tk[x] < 1) flag = is_local_max(a, fimg, zi, y, x, cur);
+      cur = row[x];
+      flag = above<kBits>(cur, a.threshold, false) && tk[x] < 1 && !beaten_nearby<kBits>(a, plane, sy, ey, y, x, cur);
     }
-    const uint32_t b = __ballot_sync(0xffffffffu, flag);
+    uint32_t b = __ballot_sync(0xffffffffu, flag);
+    for (uint32_t todo = b; todo; todo &= todo - 1) {
+      const int k = __ffs(todo) - 1, xi = w * 32 + k;
+      const double c = __shfl_sync(0xffffffffu, cur, k);
+      const int sx = max(xi - a.cr, 0), nx = min(xi + a.cr, a.C - 1) - sx + 1, n = (ey - sy + 1) * nx;
+      bool beaten = false;
+      for (int z = sz; z <= ez; ++z) {
+        const double* p = fimg + (size_t)z * a.R * a.C;
+        for (int i = lane; i < n; i += 32) {
+          const int iy = i / nx, yy = sy + iy, xx = sx + i - iy * nx;
+          const int dy = yy - y, dx = xx - xi;
+          if (dx * dx + dy * dy > a.rr) continue;
+          beaten |= above<kBits>(p[(size_t)yy * a.C + xx], c, !(yy <= y && xx <= xi));
+        }
+      }
+      if (__any_sync(0xffffffffu, beaten)) b &= ~(1u << k);
+    }
     if (lane == 0) bits[w] = b;
     cnt += __popc(b);
   }
@@ -474,7 +663,7 @@ __global__ void k_sub(const double* __restrict__ a, const double* __restrict__ b
                       double* __restrict__ out, size_t total) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
        i += (size_t)gridDim.x * blockDim.x)
-    out[i] = b ? a[i] - b[i] : a[i];
+    out[i] = a[i] - b[i];
 }
 
 // masked = (fg / sqrt(bgv <= 0.1 ? 0.1 : bgv)) * mask (fitting.py:470-497).
@@ -760,6 +949,7 @@ struct MFilter {
   double* d_io2 = nullptr;
   cudaStream_t stream = nullptr;
   int64_t launches = 0;
+  int sms = 1;                 // the device's SMs
   size_t smem_fast = 0, smem_slow = 0, smem_2d = 0;
 };
 
@@ -820,18 +1010,58 @@ int filter_run(MFilter* m, const double* d_in, int n, int memo, cudaStream_t s) 
     FCK(cudaMemsetAsync(m->d_flag, 0, sizeof(int) * n, s));
     const dim3 g(std::min(64, (npix + kThreads - 1) / kThreads), n);
     k_memo_diff<<<g, kThreads, 0, s>>>(d_in, m->d_old, npix, m->max_diff, m->d_flag);
-    k_memo_copy<<<g, kThreads, 0, s>>>(d_in, m->d_old, npix, m->d_flag);
-    m->launches += 2;
+    m->launches += 1;
+    if (!(m->separable && m->ff)) {
+      k_memo_copy<<<g, kThreads, 0, s>>>(d_in, m->d_old, npix, m->d_flag);
+      m->launches += 1;
+    }
   } else {
     FCK(cudaMemsetAsync(m->d_flag, 0x01, sizeof(int) * n, s));
   }
   if (m->separable) {
     const dim3 g((m->C + kTC - 1) / kTC, (m->R + kSlowTR - 1) / kSlowTR, n);
     if (m->ff) {
-      k_conv_fast_ff<<<dim3(m->R, n), kThreads, m->smem_fast, s>>>(d_in, m->d_tmp, m->R, m->C, m->d_wb_ff,
-                                                                  m->b0, m->nb, m->d_flag);
-      k_conv_slow_ff<<<g, dim3(kTC, kThreads / kTC), m->smem_slow, s>>>(m->d_tmp, m->d_last, m->R, m->C,
-                                                                         m->d_wa_ff, m->a0, m->na, m->d_flag);
+      // Threads and rows of a fast-axis block: those that leave the fewest
+      // lanes idle (8 outputs a lane: 4 rows of 534 pixels fill 93 % of three
+      // warps three times), but four blocks for each SM where there are so
+      // many rows.  Small blocks, as many as fit an SM: one stages its rows
+      // while another sums (32 frames of 534 x 534, 81 taps: 410 us, blocks of 352
+      // threads 460).
+      const auto smem = [&](bool two, int spread, int rb) {
+        const int next = fast_units(m->C, two) * kFastQ + m->nb - 1;
+        return (two ? sizeof(FF2) : sizeof(FF1)) * (size_t)(m->nb + rb * (fast_at(next, spread) + 1));
+      };
+      const bool two = smem(true, 2, 1) <= kSmemMax;
+      const int spread = smem(two, 2, 1) <= kSmemMax ? 2 : 31;
+      const int nu = fast_units(m->C, two);
+      const int most = (int)std::max(1LL, std::min((long long)kFastRows, (long long)m->R * n / (4 * m->sms)));
+      const auto idle = [&](int rows, int t) {   // lanes without an output, per row
+        return (double)((rows * nu + t - 1) / t * t - rows * nu) / rows;
+      };
+      int rb = 1, threads = kFastThreads;
+      for (int k = 1; k <= most && (k == 1 || smem(two, spread, k) <= kFastSmem); ++k)
+        for (int t = kFastThreads; t >= 64; t -= 32)
+          if (idle(k, t) < idle(rb, threads)) {
+            rb = k;
+            threads = t;
+          }
+      float2* tmp = reinterpret_cast<float2*>(m->d_tmp);
+      double* old = memo ? m->d_old : nullptr;
+      const dim3 gf((m->R + rb - 1) / rb, n);
+      if (two) {
+        k_conv_fast_ff<FF2><<<gf, threads, smem(two, spread, rb), s>>>(d_in, tmp, m->R, m->C, m->d_wb_ff, m->b0,
+                                                                            m->nb, m->d_flag, rb, spread, old);
+      } else {
+        k_conv_fast_ff<FF1><<<gf, threads, smem(two, spread, rb), s>>>(d_in, tmp, m->R, m->C, m->d_wb_ff, m->b0,
+                                                                            m->nb, m->d_flag, rb, spread, old);
+      }
+      // Slow-axis pass: the largest tile re-reads the least halo; a quarter
+      // of it where that makes less than two blocks for each SM.
+      const bool wide = (size_t)g.x * g.y * g.z >= 2 * (size_t)m->sms;
+      const int ny = wide ? kSlowTR / kSlowQ : kSlowTR / kSlowQ / 4, tr = ny * kSlowQ;
+      k_conv_slow_ff<<<dim3(g.x, (m->R + tr - 1) / tr, n), dim3(kTC / 2, ny),
+                       sizeof(FF2) * (size_t)(m->na + (tr + m->na - 1) * (kTC / 2)), s>>>(
+          tmp, m->d_last, m->R, m->C, m->d_wa_ff, m->a0, m->na, m->d_flag);
     } else {
       k_conv_fast<<<dim3(m->R, n), kThreads, m->smem_fast, s>>>(d_in, m->d_tmp, m->R, m->C, m->d_wb,
                                                                m->b0, m->nb, m->d_flag);
@@ -910,6 +1140,8 @@ MFilter* filter_create(const double* psf, double max_diff, int R, int C) {
   m->R = R;
   m->C = C;
   m->max_diff = max_diff > 0.0 ? max_diff : 0.0;
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev);
   m->h_rc.assign(psf, psf + (size_t)R * C);
   const std::vector<double>& p = m->h_rc;
   const PsfTaps taps = analyze_psf(p, R, C);
@@ -968,8 +1200,9 @@ MFilter* filter_create(const double* psf, double max_diff, int R, int C) {
          cudaMemcpy(m->d_w2, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice) == cudaSuccess;
   }
   ok = ok && cudaFuncSetAttribute(k_conv_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) == cudaSuccess &&
-       cudaFuncSetAttribute(k_conv_fast_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) == cudaSuccess &&
-       cudaFuncSetAttribute(k_conv_slow_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) == cudaSuccess &&
+       cudaFuncSetAttribute(k_conv_fast_ff<FF1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax + 64) == cudaSuccess &&
+       cudaFuncSetAttribute(k_conv_fast_ff<FF2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) == cudaSuccess &&
+       cudaFuncSetAttribute(k_conv_slow_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlowSmemMax) == cudaSuccess &&
        cudaFuncSetAttribute(k_conv_slow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) == cudaSuccess &&
        cudaFuncSetAttribute(k_conv_2d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) == cudaSuccess &&
        cudaMalloc(&m->d_io, sizeof(double) * (size_t)R * C) == cudaSuccess &&
@@ -1110,7 +1343,8 @@ int maxima_mark(Maxima* h, const double* d_img, int n, cudaStream_t s) {
   const LMax a = lmax_args(h, d_img, n);
   const int warps_per_block = kThreads / 32;
   const int blocks = (a.nrows + warps_per_block - 1) / warps_per_block;
-  k_lmax_mark<<<blocks, kThreads, 0, s>>>(a);
+  if (a.threshold >= 0.0) k_lmax_mark<true><<<blocks, kThreads, 0, s>>>(a);
+  else k_lmax_mark<false><<<blocks, kThreads, 0, s>>>(a);
   k_lmax_scan<<<1, 1024, 0, s>>>(h->d_rowcnt, h->d_rowoff, a.nrows, h->Z * h->R, n, h->d_fcount);
   h->launches += 2;
   FCK(cudaGetLastError());
@@ -1930,11 +2164,13 @@ int saFinderEstimateBackground(void* fh, const double* fit, const double* bg_est
   }
   const double* f = finder_input(h, fit, on_device, &h->d_fit, n);
   if (fit && !f) return -1;
-  k_sub<<<grid_for(total), kThreads, 0, h->stream>>>(h->d_image, f, h->d_a, total);
-  h->launches += 1;
-  FCK(cudaGetLastError());
+  if (f) {
+    k_sub<<<grid_for(total), kThreads, 0, h->stream>>>(h->d_image, f, h->d_a, total);
+    h->launches += 1;
+    FCK(cudaGetLastError());
+  }
   const int64_t l0 = h->bg->launches;
-  if (filter_run(h->bg, h->d_a, n, 1, h->stream)) return -1;
+  if (filter_run(h->bg, f ? h->d_a : h->d_image, n, 1, h->stream)) return -1;
   h->launches += h->bg->launches - l0;
   h->d_background = h->bg->d_last;
   return 0;

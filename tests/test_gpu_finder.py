@@ -575,3 +575,74 @@ def test_spliner_find_fit_loop_matches_oracle():
     zr = numpy.array([spline.rescaleZ(z) for z in ref["z"]])
     ok = (near < 1e-4) & (numpy.abs(got["z"][j] - zr) < 1e-3)
     assert numpy.mean(ok) >= 0.9
+
+
+@pytest.mark.parametrize("shape,sigma,n", [((41, 53), 2.0, 1), ((7, 9), 1.0, 3), ((90, 31), 1.5, 5), ((129, 1), 1.0, 2),
+                                           ((1, 130), 1.0, 2), ((300, 257), 8.0, 12), ((96, 24001), 2.0, 1)])
+def test_float_pair_passes_over_shapes(monkeypatch, shape, sigma, n):
+    """The float-pair passes at odd widths, rows shorter than the taps, one
+    to many frames (both heights of the slow-axis tile) and rows that fill
+    the shared memory one output at a time, against the FP64 passes to
+    1e-13 of the magnitude; zeros, negative values and values beyond the
+    floats' usual range among the inputs, and the kept image of a memoised
+    filter used only while the frame stays within max_diff."""
+    import ctypes
+    import torch
+    from sa_gb300 import loadclib
+    lib = loadclib.load()
+    rng = numpy.random.default_rng(shape[0] + shape[1])
+    ax = [numpy.exp(-0.5 * ((numpy.arange(m) - m // 2) / sigma) ** 2) * (abs(numpy.arange(m) - m // 2) <= 5 * sigma)
+          for m in shape]
+    psf = numpy.roll(ax[0][:, None] * ax[1][None, :], (-(shape[0] // 2), -(shape[1] // 2)), (0, 1))
+    psf = numpy.ascontiguousarray(psf / psf.sum())
+    img = rng.uniform(-200.0, 5000.0, (n,) + shape)
+    img[rng.random(img.shape) < 0.1] = 0.0
+    img[rng.random(img.shape) < 0.05] *= 2.0 ** -70
+    outs = []
+    for fp64 in ("0", "1"):
+        monkeypatch.setenv("SA_FINDER_FP64", fp64)
+        h = lib.saFilterCreate(psf, 1.0e-3, shape[0], shape[1], 0)
+        assert h, loadclib.last_error()
+        d = torch.from_numpy(img).cuda()
+        got = []
+        for step in range(3):   # first, unchanged (kept), changed in its last frame
+            if step == 2:
+                d[n - 1, shape[0] - 1, shape[1] - 1] += 100.0
+            o = torch.empty_like(d)
+            torch.cuda.synchronize()
+            assert lib.saFilterConvolveDevice(h, d.data_ptr(), n, 1, o.data_ptr()) == 0
+            torch.cuda.synchronize()
+            got.append(o.cpu().numpy())
+        lib.saFilterCleanup(h)
+        outs.append(got)
+    scale = numpy.abs(outs[1][0]).max()
+    for a, b in zip(*outs):
+        assert numpy.abs(a - b).max() <= 1e-13 * scale
+    for got in outs:
+        assert numpy.array_equal(got[0], got[1])
+        assert not numpy.array_equal(got[1][n - 1], got[2][n - 1])
+
+
+@pytest.mark.parametrize("threshold", [-3.0, 0.0, 2.0])
+@pytest.mark.parametrize("shape,radius,planes", [((12, 31), 5.0, 1), ((33, 32), 1.0, 1), ((40, 65), 0.4, 1),
+                                                 ((35, 97), 3.3, 3), ((64, 64), 70.0, 2)])
+def test_local_maxima_over_thresholds_and_radii(threshold, shape, radius, planes):
+    """Local maxima against the oracle: comparisons on bit patterns (threshold
+    0 and above) and on doubles (below), ties, infinities, NaN and signed
+    zeros, radii from under a pixel to beyond the image, several planes."""
+    from sa_gb300 import ia_utilities_c
+    rng = numpy.random.default_rng(int(10 * radius) + shape[1])
+    imgs = [numpy.round(rng.normal(0.0, 4.0, shape)) for _ in range(planes)]
+    for im in imgs:
+        im[rng.random(shape) < 0.02] = numpy.nan
+        im[rng.random(shape) < 0.01] = numpy.inf
+        im[rng.random(shape) < 0.01] = -numpy.inf
+        im[rng.random(shape) < 0.05] = -0.0
+        im[rng.random(shape) < 0.02] = -numpy.nan
+    kw = dict(margin=1, radius=radius, threshold=threshold, z_range=min(1, planes - 1), z_values=list(range(planes)))
+    g, o = ia_utilities_c.MaximaFinder(**kw), F.MaximaFinder(**kw)
+    for _ in range(2):
+        a, b = g.findMaxima(imgs), o.findMaxima(imgs)
+        for u, v in zip(a[:3], b[:3]):
+            assert numpy.array_equal(numpy.asarray(u), numpy.asarray(v))
+    g.cleanup()
