@@ -36,8 +36,8 @@ static cudaError_t mp_limits() {
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)a.sharedSizeBytes);
     if (e != cudaSuccess) return e;
+    if (fn == (const void*)k_mp_sweep) g_max_smem = max_smem - (int)a.sharedSizeBytes;
   }
-  g_max_smem = max_smem;
   done = true;
   return cudaSuccess;
 }
