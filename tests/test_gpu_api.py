@@ -216,3 +216,28 @@ def test_escape_rollback_path_is_exact():
     assert outs[1][1]["reruns"] > 0
     for p in ["x", "y", "height", "status", "iterations"]:
         assert numpy.array_equal(outs[0][0][p], outs[1][0][p]), p
+
+
+@pytest.mark.parametrize("counts", [(0, 1, 129, 128, 0, 3), (127,), (0, 0, 5)])
+def test_result_rows_are_the_peak_properties(counts):
+    """saGetResultsBatch's rows (made on the device) equal the properties
+    read one by one, for frames with no peaks, one, and either side of a
+    block of 128."""
+    from sa_gb300 import engine
+    rng = numpy.random.default_rng(sum(counts))
+    shape = (60, 75)
+    fit = engine.BatchFitter("2d", shape, len(counts), roi_size=8, sigma_range=[0.5, 3.0])
+    peaks = [dict(x=rng.uniform(10.0, 65.0, n), y=rng.uniform(10.0, 50.0, n), z=numpy.zeros(n),
+                  background=numpy.full(n, 20.0), height=rng.uniform(100.0, 300.0, n),
+                  xsigma=rng.uniform(0.8, 2.0, n), ysigma=rng.uniform(0.8, 2.0, n)) for n in counts]
+    images = rng.poisson(30.0, (len(counts),) + shape).astype(numpy.float32)
+    fit.load(images, numpy.full_like(images, 20.0), peaks, "hdf5")
+    fit.fit(5)
+    values, ints = fit.results_fast()
+    assert values.shape[0] == sum(counts)
+    columns = ("x", "y", "z", "height", "background", "xsigma", "ysigma", "error")
+    ref = fit.results(columns)
+    for k, name in enumerate(columns):
+        assert numpy.array_equal(values[:, k], ref[name], equal_nan=True), name
+    assert numpy.array_equal(ints[:, 0], ref["status"]) and numpy.array_equal(ints[:, 1], ref["iterations"])
+    fit.close()
