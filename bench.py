@@ -368,7 +368,7 @@ def run_ours(args, rank, world, local_rank):
         step_e2e()
     ms_e2e = timed(step_e2e, args.steps)
     h2d = images.nbytes + bgs.nbytes + rows.nbytes + counts.nbytes
-    d2h = int(units * 128)
+    d2h = int(units * 72)   # eight doubles and two 32-bit words a peak
 
     # plain one-frame-per-launch fitter (host-driven sweep loop), bounded sample
     plain = None
@@ -1069,9 +1069,9 @@ def run_mp_report(args, pool):
             "batch_cpu_localizations_per_s": n_cpu_batch / cpu_batch_s, "batch_cpu_frames": ncpu,
             "batch_cpu_cores": getattr(pool, "_processes", None),
             "batch_timing": "best of 2 fits after a warm-up fit, host images to results",
-            "note": "a frame is one CTA: batches of consecutive groups whose grown ROIs do not overlap "
-                    "step at once (up to 8 for a lone frame, 2-3 when many frames share the GPU), committed "
-                    "in index order (the reference's sweep order); frames run in parallel (mpDoFitBatch); "
+            "note": "a frame is one CTA, or a cluster of up to 8 while SMs are idle: batches of consecutive "
+                    "groups whose grown ROIs do not overlap step at once (up to 16 for a lone frame, 2-3 when "
+                    "many frames share the GPU), committed in index order (the reference's sweep order); frames run in parallel (mpDoFitBatch); "
                     "FP64 throughout"}
 
 
