@@ -299,7 +299,7 @@ void mpDaoNewPeaks(saMPFit *mp_fit, double *peak_params, char *p_type, int n_pea
  * saNewBackgrounds on each fit_data[i], new peaks of every frame in
  * channel 0's coordinates (counts[f] rows each, frames one after another;
  * the frames' images just loaded), then doFit's sweeps for every frame at
- * once (one warp per frame); results per channel with saGetResultsBatch.
+ * once; results per channel with saGetResultsBatch.
  * Return 0 (mpDoFitBatch: the number of sweeps) or -1 (saGetLastError). */
 int mpSetFrames(saMPFit *mp_fit, int n_frames, int peaks_capacity);
 int mpNewPeaksBatch(saMPFit *mp_fit, const double *peak_params, const int32_t *counts, const char *p_type);
