@@ -193,8 +193,8 @@ template <typename T>
 cudaError_t Launch<T>::new_peaks_finder(const ModelCfg& cfg, const FrameSet<T>& fs, const int* slots,
                                         const int* frame_first, const int* frame_n, int nframes,
                                         size_t warp_smem, cudaStream_t s) {
-  const int g = (nframes * 32 + aux_block(cfg) - 1) / aux_block(cfg);
-  k_newpeaks_finder<T><<<g, aux_block(cfg), warp_smem, s>>>(cfg, fs, slots, frame_first, frame_n, nframes);
+  if (nframes <= 0) return cudaSuccess;
+  k_newpeaks_finder<T><<<nframes, aux_block(cfg), warp_smem, s>>>(cfg, fs, slots, frame_first, frame_n);
   return cudaGetLastError();
 }
 

@@ -241,3 +241,37 @@ def test_result_rows_are_the_peak_properties(counts):
         assert numpy.array_equal(values[:, k], ref[name], equal_nan=True), name
     assert numpy.array_equal(ints[:, 0], ref["status"]) and numpy.array_equal(ints[:, 1], ref["iterations"])
     fit.close()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("n,spread", [(1, 1.0), (8, 1.0), (9, 1.0), (60, 1.0), (40, 0.25), (23, 0.05)])
+def test_finder_peaks_heights_in_input_order(precision, n, spread):
+    """The height of a "finder" peak is estimated on the image that holds
+    the earlier ones: sparse, crowded and coinciding peaks (batches of 8, 8
+    and a remainder, and of 1 where every ROI overlaps), some outside the
+    frame, against the oracle's one after another."""
+    import os
+    import sys
+    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    from oracle.oracle import OracleFitter
+    from sa_gb300 import dao_fit_c
+    rng = numpy.random.default_rng(n)
+    ny, nx = 90, 101
+    x = 0.5 * nx + spread * rng.uniform(-0.5, 0.5, n) * (nx - 8)
+    y = 0.5 * ny + spread * rng.uniform(-0.5, 0.5, n) * (ny - 8)
+    image = gauss_image((ny, nx), [(a, b, 300.0, 1.3) for a, b in zip(x, y)], 20.0)
+    peaks = dict(x=numpy.round(x), y=numpy.round(y), z=numpy.zeros(n), sigma=numpy.full(n, 1.3))
+    out = []
+    for f in (OracleFitter("2d", (ny, nx), roi_size=10, sigma_range=[0.5, 3.0]),
+              dao_fit_c.MultiFitter2D(roi_size=10, sigma_range=[0.5, 3.0], precision=precision)):
+        if not isinstance(f, OracleFitter):
+            f.initializeC(image)
+        f.newImage(image)
+        f.newBackground(numpy.full((ny, nx), 20.0))
+        f.newPeaks(peaks, "finder")
+        out.append({k: f.getPeakProperty(k) for k in ("height", "status")})
+        f.cleanup(verbose=False)
+    assert numpy.array_equal(out[1]["status"], out[0]["status"])
+    # the fit image in 36 fractional bits and FP32 shapes against doubles
+    tol = 1e-9 if precision == 64 else 1e-5
+    assert numpy.abs(out[1]["height"] - out[0]["height"]).max() <= tol * numpy.abs(out[0]["height"]).max()
