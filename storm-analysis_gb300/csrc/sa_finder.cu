@@ -166,22 +166,43 @@ k_conv_slow(const double* __restrict__ in, double* __restrict__ out, int R, int 
 //
 // The FP64 pipe (an instruction of a warp takes a scheduler 64 cycles) is
 // kept off the path as far as the formats allow: an input is split with
-// integer operations (nearest float and remainder; values outside the floats'
-// normal range take the FP64 conversions), the first pass hands its pairs to
-// the second as they are, and only the last sum becomes a double.
+// integer operations (nearest float, ties to even, and remainder: the bits of
+// the two conversions; values outside the floats' normal range take those),
+// and between the passes a pair is rounded to a double's 53 bits as a pair.
+// Only the last sum becomes a double.
 __device__ __forceinline__ float2 ff_split(double v) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
   if (e - 963u < 186u) {   // 2^-60 <= |v| < 2^126: both floats are normal or zero
-    const unsigned long long r = b + 0x10000000ull;         // the upper 23 bits, rounded (half up)
+    const unsigned half = 0x0fffffffu + ((unsigned)(b >> 29) & 1u);
+    const unsigned long long r = b + half;                                   // the upper 23 bits, rounded
     const unsigned hi = (unsigned)(r >> 32) & 0x7fffffffu;
     const float h = __uint_as_float(((hi - (896u << 20)) << 3) | ((unsigned)r >> 29) | ((unsigned)(b >> 32) & 0x80000000u));
-    const int rem = (int)((unsigned)r & 0x1fffffffu) - 0x10000000;          // v - h in units of 2^(e - 1075)
-    const float unit = __uint_as_float(((e - 948u) << 23) | ((unsigned)(b >> 32) & 0x80000000u));
-    return make_float2(h, __int2float_rn(rem) * unit);
+    const int rem = (int)((unsigned)r & 0x1fffffffu) - (int)half;            // |v| - |h| in units of 2^(e - 1075)
+    return make_float2(h, __int2float_rn((long long)b < 0 ? -rem : rem) * __uint_as_float((e - 948u) << 23));
   }
   const float h = __double2float_rn(v);
   return make_float2(h, __double2float_rn(v - (double)h));
+}
+
+// ff_split of the double nearest to the pair's sum.  A pair holds more bits
+// than a double where its low word lies far enough below the high one; the
+// second pass takes what a double holds, as if the first had stored doubles
+// (without this one background pixel in 8,000 moved by up to 1e-14 of its
+// value, and what the find / fit loop fits to it by 1e-9).  The low word is
+// rounded by adding and taking away a power of two whose last bit is the
+// double's; pairs that are not normalised, or near the ends of the range,
+// take the conversions.  The pass over 32 frames of
+// 534 x 534, 81 taps: 423 us, 410 without.
+__device__ __forceinline__ float2 ff_as_double(float2 v) {
+  const unsigned h = __float_as_uint(v.x), l = __float_as_uint(v.y);
+  unsigned a = (h >> 23) & 0xffu;
+  if (a - 60u < 190u && __fadd_rn(v.x, v.y) == v.x) {
+    if ((h & 0x7fffffu) == 0u && ((h ^ l) >> 31)) a--;   // the sum lies below the power of two v.x
+    const float big = __uint_as_float((a - 29u) << 23), c = copysignf(big, v.y);
+    return make_float2(v.x, fabsf(v.y) < big ? __fsub_rn(__fadd_rn(v.y, c), c) : v.y);
+  }
+  return ff_split((double)v.x + (double)v.y);
 }
 
 __host__ __device__ __forceinline__ int fast_units(int C, bool two) {
@@ -269,7 +290,7 @@ __device__ __forceinline__ FF2 ff_weight(float2 w, FF2) { return FF2{f2(w.x, w.x
 // chain of additions.  Each sum keeps the order of its taps.  What bounds it is
 // the FP32 pipe, 15 operations a tap: 32 frames of 534 x 534 and 81 taps take
 // it 300 us, the slow-axis pass 370 and the fast-axis pass (which also splits
-// the doubles and keeps the image) 410; 490 and 440 + 26 before.
+// the doubles, rounds its sums and keeps the image) 423; 490 and 440 + 26 before.
 template <int NQ, typename V, typename X>
 __device__ __forceinline__ void ff_sums(const V* ws, int na, X x, V* sum) {
   V ring[NQ];   // ring[(q - i) mod NQ] = x(na - 1 - i + q)
@@ -291,12 +312,12 @@ __device__ __forceinline__ void ff_sums(const V* ws, int na, X x, V* sum) {
 }
 
 __device__ __forceinline__ void ff_store(FF1 v, float2* o, int c, int, int C) {
-  if (c < C) o[c] = v.v;
+  if (c < C) o[c] = ff_as_double(v.v);
 }
 __device__ __forceinline__ void ff_store(FF2 v, float2* o, int c, int half, int C) {
   const float2 h = f2_get(v.h), l = f2_get(v.l);
-  if (c < min(half, C)) o[c] = make_float2(h.x, l.x);
-  if (c < half && c + half < C) o[c + half] = make_float2(h.y, l.y);
+  if (c < min(half, C)) o[c] = ff_as_double(make_float2(h.x, l.x));
+  if (c < half && c + half < C) o[c + half] = ff_as_double(make_float2(h.y, l.y));
 }
 
 // kFastQ outputs (FF2: two times kFastQ, half a row apart) a thread, rb rows
@@ -1025,8 +1046,8 @@ int filter_run(MFilter* m, const double* d_in, int n, int memo, cudaStream_t s) 
       // lanes idle (8 outputs a lane: 4 rows of 534 pixels fill 93 % of three
       // warps three times), but four blocks for each SM where there are so
       // many rows.  Small blocks, as many as fit an SM: one stages its rows
-      // while another sums (32 frames of 534 x 534, 81 taps: 410 us, blocks of 352
-      // threads 460).
+      // while another sums (32 frames of 534 x 534, 81 taps, before the sums
+      // were rounded: 410 us, blocks of 352 threads 460).
       const auto smem = [&](bool two, int spread, int rb) {
         const int next = fast_units(m->C, two) * kFastQ + m->nb - 1;
         return (two ? sizeof(FF2) : sizeof(FF1)) * (size_t)(m->nb + rb * (fast_at(next, spread) + 1));

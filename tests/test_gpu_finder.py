@@ -646,3 +646,61 @@ def test_local_maxima_over_thresholds_and_radii(threshold, shape, radius, planes
         for u, v in zip(a[:3], b[:3]):
             assert numpy.array_equal(numpy.asarray(u), numpy.asarray(v))
     g.cleanup()
+
+
+def _split(v):
+    h = v.astype(numpy.float32)
+    return h, (v - h.astype(numpy.float64)).astype(numpy.float32)
+
+
+def _fma(a, b, c):
+    return (a.astype(numpy.float64) * b.astype(numpy.float64) + c.astype(numpy.float64)).astype(numpy.float32)
+
+
+def _float_pair_pass(img, taps, first, axis):
+    """One pass of the separable filter in float pairs, doubles in and out."""
+    xh, xl = _split(img)
+    wh, wl = _split(taps)
+    sh, sl = numpy.zeros_like(xh), numpy.zeros_like(xl)
+    for i in range(taps.size):
+        ah, al = numpy.roll(xh, first + i, axis=axis), numpy.roll(xl, first + i, axis=axis)
+        p = wh[i] * ah
+        e = _fma(wl[i], ah, _fma(wh[i], al, _fma(wh[i], ah, -p)))
+        s = sh + p
+        v = s - sh
+        t = ((sh - (s - v)) + (p - v)) + sl + e
+        sh = s + t
+        sl = t - (sh - s)
+    return sh.astype(numpy.float64) + sl.astype(numpy.float64)
+
+
+@pytest.mark.parametrize("shape,sigma", [((130, 131), 8.0), ((96, 257), 1.0), ((7, 9), 1.0), ((129, 1), 1.0),
+                                         ((4, 24001), 2.0)])
+def test_passes_exchange_doubles(shape, sigma):
+    """The float-pair passes bit for bit as they are defined: each takes
+    doubles (split to nearest, ties to even) and gives doubles, so the
+    second pass sees 53 bits of the first one's sums.  Two outputs at a time
+    and (24,001 columns) one; values half way between two floats, signed
+    zeros, and values outside the floats' normal range among the inputs."""
+    from sa_gb300 import loadclib
+    lib = loadclib.load()
+    rng = numpy.random.default_rng(shape[1])
+    psf = numpy.ascontiguousarray(F.recenter_psf(F.gaussian_psf(shape, sigma)))
+    out = numpy.zeros(5, dtype=numpy.int32)
+    u, v = numpy.zeros(shape[0]), numpy.zeros(shape[1])
+    assert lib.saFilterAnalyze(psf, shape[0], shape[1], out, u.ctypes.data_as(ctypes.c_void_p),
+                               v.ctypes.data_as(ctypes.c_void_p)) == 0
+    assert out[0] == 1
+    img = rng.uniform(-200.0, 5000.0, shape)
+    ties = rng.random(shape) < 0.2
+    img[ties] = 2.0 ** 24 + 2.0 * rng.integers(0, 500, ties.sum()) + 1.0
+    img[rng.random(shape) < 0.05] = -0.0
+    img[rng.random(shape) < 0.02] *= 2.0 ** -64
+    ref = _float_pair_pass(img, v[:out[2]], int(out[4]), 1)
+    ref = _float_pair_pass(ref, u[:out[1]], int(out[3]), 0)
+    h = lib.saFilterCreate(psf, 0.0, shape[0], shape[1], 0)
+    assert h, loadclib.last_error()
+    got = numpy.zeros(shape)
+    assert lib.saFilterConvolve(h, img, got) == 0
+    lib.saFilterCleanup(h)
+    assert numpy.array_equal(got, ref)
