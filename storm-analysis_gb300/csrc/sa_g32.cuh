@@ -31,6 +31,15 @@
 
 namespace sa {
 
+// Barrier ID of `count` threads of the CTA (whole warps); arrive: without
+// waiting for the others.
+__device__ __forceinline__ void bar_sync(int id, int count) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int count) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
 enum { ACT_EVAL = 0, ACT_CONTINUE = 1, ACT_BREAK = 2, ACT_BREAK_ADDED = 3, ACT_ESCAPE = 4 };
 
 // Per-axis Jacobian factors of pass 1 in tab1 (ff pairs, stride ts):
@@ -805,9 +814,7 @@ template <int M, int NW>
 __device__ inline void g32_prologue(const ModelCfg& cfg, const FrameSet<float>& fs, const PeakRec* recp,
                                     WarpWS<float>& ws, int tid) {
   const int lane = tid & 31, w = tid >> 5;
-  auto sync = []() {
-    asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
-  };
+  auto sync = []() { bar_sync(1, NW * 32); };
   if (w == 0) {
     if (lane < 8) {
       const double2 v = __ldcg(reinterpret_cast<const double2*>(recp) + lane);
@@ -984,9 +991,14 @@ __device__ bool lm_step_g32(const ModelCfg& cfg, const FrameSet<float>& fs, long
         else if (dbl_gt_pos(lambda, LAMBDA_MIN)) lambda = LAMBDA_DOWN * lambda;
         act = ACT_BREAK_ADDED;
       }
+      // The next trial writes the slots and may write the tables (the solver's
+      // scratch) that the other warps read for the change: not before they
+      // are done.  They are by now, or warp 0 would wait for them above.
+      if (is_delta) bar_sync(2, TEAM);
     } else if (is_delta) {
 #pragma unroll 1
       for (int p = tid - 32; p < cfg.nroi; p += TEAM - 32) g32_pixel_change(cfg, fs, ws, p);
+      bar_arrive(2, TEAM);
     }
   }
 

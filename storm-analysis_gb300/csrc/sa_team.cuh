@@ -22,11 +22,6 @@
 
 namespace sa {
 
-// Barrier ID of `count` threads of the CTA (whole warps).
-__device__ __forceinline__ void bar_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-
 // A team step's view of the workspace: the warp step's arrays and tables (b)
 // and what only the team keeps.
 template <typename T>
@@ -526,18 +521,19 @@ __device__ inline double team_trial_sum(const ModelCfg& cfg, const TeamWS<float>
   return ff_to_double(warp_sum_ffv(s1)) + warp_sum_ff(s2);
 }
 
-// The trial's contribution at pixel p of its ROI (image pixel k).
+// The trial's contribution (height h, background bg) at pixel p of its ROI
+// (image pixel k).
 __device__ __forceinline__ void team_trial_contrib(const ModelCfg& cfg, const FrameSet<double>& fs,
-                                                   const TeamWS<double>& ws, const PeakRec& t, const SplinePos&,
+                                                   const TeamWS<double>& ws, double h, double bg, const SplinePos&,
                                                    int p, int, int, long long k, Q2& cf, Q2& cb) {
   const double rq = ws.b.R[p];
-  cf = quant_t<double>(contrib_f(t.p[PH], ws.b.psf[p], rq));
-  cb = quant_t<double>(contrib_bg(t.p[PBG], rq, __ldg(fs.scmos + k)));
+  cf = quant_t<double>(contrib_f(h, ws.b.psf[p], rq));
+  cb = quant_t<double>(contrib_bg(bg, rq, __ldg(fs.scmos + k)));
 }
 __device__ __forceinline__ void team_trial_contrib(const ModelCfg& cfg, const FrameSet<float>& fs,
-                                                   const TeamWS<float>& ws, const PeakRec& t, const SplinePos& s,
+                                                   const TeamWS<float>& ws, double h, double bg, const SplinePos& s,
                                                    int p, int rx, int ry, long long k, Q2& cf, Q2& cb) {
-  spl32_contrib(spline_value_ff(cfg, fs.aij, ws.b, s, rx, ry), ff_from_double(t.p[PH]), ff_from_double(t.p[PBG]),
+  spl32_contrib(spline_value_ff(cfg, fs.aij, ws.b, s, rx, ry), ff_from_double(h), ff_from_double(bg),
                 ws.b.R[p], __ldg(fs.scmos + k), cf, cb);
 }
 
@@ -670,6 +666,11 @@ __device__ bool team_step(const ModelCfg& cfg, const FrameSet<T>& fs, long long 
     fail = false;
 #pragma unroll 1
     for (int p = tid; p < cfg.nroi; p += NT) team_pixel_trial(cfg, fs, fbase, ws, orig, t, s, delta, p, fail);
+    // Past this barrier warp 0 may make the next trial of t: what the other
+    // warps still need of it is read before.  (The solve writes none of the
+    // tables they read; the next trial's are made behind the barrier above.)
+    const bool home = cax == orig.xi && cay == orig.yi && t.xi == orig.xi && t.yi == orig.yi;
+    const double h = t.p[PH], bg = t.p[PBG];
     fail = __syncthreads_or(fail);
     if (wid == 0) {
       const double dev = team_trial_sum(cfg, ws, delta, lane);
@@ -705,13 +706,13 @@ __device__ bool team_step(const ModelCfg& cfg, const FrameSet<T>& fs, long long 
       }
     } else if constexpr (sizeof(T) == 4) {
       // the trial's change of the fit image, while warp 0 decides
-      if (cax == t.xi && cay == t.yi && t.xi == orig.xi && t.yi == orig.yi) {
+      if (home) {
 #pragma unroll 1
         for (int p = tid - 32; p < cfg.nroi; p += NT - 32) {
           int rx, ry;
           roi_rc(ws.b.roi, p, rx, ry);
           Q2 cf, cb;
-          team_trial_contrib(cfg, fs, ws, t, s, p, rx, ry, pix_index(cfg, t.xi, t.yi, rx, ry), cf, cb);
+          team_trial_contrib(cfg, fs, ws, h, bg, s, p, rx, ry, pix_index(cfg, orig.xi, orig.yi, rx, ry), cf, cb);
           ws.q1f[p] = cf.h - ws.q0f[p];
           ws.q1b[p] = cb.h - ws.q0b[p];
         }
@@ -737,7 +738,7 @@ __device__ bool team_step(const ModelCfg& cfg, const FrameSet<T>& fs, long long 
         cb = Q2{ws.q1b[p], 0};
       } else {
         Q2 of, ob;
-        team_trial_contrib(cfg, fs, ws, t, s, p, rx, ry, k0, cf, cb);
+        team_trial_contrib(cfg, fs, ws, t.p[PH], t.p[PBG], s, p, rx, ry, k0, cf, cb);
         team_start_contrib(fs, ws, orig, p, ws.b.R[p], __ldg(fs.scmos + k0), of, ob);
         cf = q_sub(cf, of);
         cb = q_sub(cb, ob);
@@ -752,7 +753,7 @@ __device__ bool team_step(const ModelCfg& cfg, const FrameSet<T>& fs, long long 
       atomicAdd(fs.cnt + fbase + k0, -1);
       if (added_end) {
         const long long k1 = pix_index(cfg, t.xi, t.yi, rx, ry);
-        team_trial_contrib(cfg, fs, ws, t, s, p, rx, ry, k1, cf, cb);
+        team_trial_contrib(cfg, fs, ws, t.p[PH], t.p[PBG], s, p, rx, ry, k1, cf, cb);
         acc_red<W>(fs.f, fbase + k1, cf, +1);
         acc_red<W>(fs.bg, fbase + k1, cb, +1);
         atomicAdd(fs.cnt + fbase + k1, 1);

@@ -71,3 +71,57 @@ def test_team_steps_over_roi_sizes(cfg, roi):
         st = parity.compare(concat(fit_workload_gpu(wl, [0], precision)), ref)
         assert st["status_agree"] >= 0.999, (precision, st)
         assert parity.within_tolerance(st, min_fraction=0.999), (precision, st)
+
+
+def wild_workload(cfg, seed, frames=2, n=60):
+    """Starts up to 6 px off, some at the frame's edge, heights off by up to
+    e^2: trials are rejected by the dozen, and by the check of the margin."""
+    from sa_gb300 import synth
+    wl = synth.make_workload(cfg, frames=frames, nx=96, ny=90, seed=seed, n_emitters=n)
+    rng = numpy.random.default_rng(seed)
+    for g in wl["guesses"]:
+        m = g["x"].size
+        g["x"] = numpy.clip(g["x"] + rng.uniform(-6.0, 6.0, m), 12.0, 84.0)
+        g["y"] = numpy.clip(g["y"] + rng.uniform(-6.0, 6.0, m), 12.0, 78.0)
+        g["height"] = g["height"] * numpy.exp(rng.uniform(-2.0, 2.0, m))
+    return wl
+
+
+def model_fitter(wl, precision, **extra):
+    from sa_gb300 import cubic_fit_c, engine
+    kw = dict(wl["fitter"])
+    model = kw.pop("model")
+    spl = kw.pop("spline", None)
+    if spl is not None:
+        kw["spline"] = cubic_fit_c.SplinePSF(coeff=spl["coeff"])
+    kw.update(extra)
+    return engine.BatchFitter(model, (wl["ny"], wl["nx"]), len(wl["images"]), rqe=wl["rqe"],
+                              scmos_cal=wl["scmos_cal"], precision=precision, **kw)
+
+
+def fit_rows(fit, wl, sweeps):
+    """Result rows, integers and what each counter rose by."""
+    before = fit.counters()
+    fit.load(numpy.stack(wl["images"]), numpy.stack(wl["backgrounds"]), wl["guesses"], "hdf5")
+    fit.fit(sweeps)
+    values, ints = fit.results_fast()
+    return numpy.array(values), numpy.array(ints), fit.counters() - before
+
+
+@pytest.mark.parametrize("cfg,roi", [(3, None), (0, 10), (0, 20), (1, 20), (2, None)])
+def test_rejected_trials_do_not_reach_their_successors(cfg, roi):
+    """While a team's first warp decides a trial the others prepare its
+    write-back; after a rejection it makes the next trial, which may lie
+    anywhere.  ROIs of one and several pixels a thread, repeated: one result
+    and one set of counters."""
+    wl = wild_workload(cfg, 70 + cfg)
+    fit = model_fitter(wl, 32, **({} if roi is None else dict(roi_size=roi)))
+    assert fit.clib.saSetTailPeaks(fit.h, 0) == 0
+    first = fit_rows(fit, wl, 100)
+    n_dposv, n_iter, n_lost, n_margin, n_neg_fi, n_neg_height, _, n_non_decr, _ = first[2]
+    assert n_margin > 0 and n_neg_height > 0 and n_non_decr > 0
+    for _ in range(30):
+        again = fit_rows(fit, wl, 100)
+        for a, b in zip(first, again):
+            assert numpy.array_equal(a, b, equal_nan=True)
+    fit.close()
