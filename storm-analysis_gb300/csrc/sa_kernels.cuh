@@ -1414,9 +1414,10 @@ __global__ void __launch_bounds__(S::THREADS)
       S::template prologue<S::THREADS>(cfg, fs, fs.pk + base + li, ws, tid);
       __syncthreads();
       S::step(cfg, fs, fbase, fs.pk + base + li, true, 0, ws, tc, fs.stepctr + (size_t)(base + li) * NCOUNTERS, tid);
+      // before the barrier: behind it the next prologue clears the counters
+      if (wid == 0 && lane < NCOUNTERS) loc += reinterpret_cast<const int*>(S::view(ws).scratch)[lane];
       __threadfence();
       __syncthreads();
-      if (wid == 0 && lane < NCOUNTERS) loc += reinterpret_cast<const int*>(S::view(ws).scratch)[lane];
     }
     if (wid == 0) {
       const bool more = tail_end_sweep(cfg, fs, c, base, fbase, nrun, loc, wr, lane);
