@@ -514,7 +514,7 @@ __device__ __forceinline__ bool beaten_nearby(const LMax& a, const double* p, in
 // What passes the look at its neighbours is searched by the whole warp, a
 // lane per pixel of the search box: a lane of its own waited for one load
 // after another (32 frames of 534 x 534: 370 us so, 127 now).
-// kBits: threshold >= 0.
+// kBits: threshold >= 0, and not -0.0.
 template <bool kBits>
 __global__ void k_lmax_mark(LMax a) {
   const int warp = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
@@ -1302,7 +1302,7 @@ LMax lmax_args(const Maxima* h, const double* d_img, int n) {
   a.rr = (int)(h->radius * h->radius);
   a.cr = (int)std::ceil(h->radius);
   a.radius = h->radius;
-  a.threshold = h->threshold;
+  a.threshold = h->threshold + 0.0;   // -0.0 as 0.0: above<true> compares the bits
   return a;
 }
 

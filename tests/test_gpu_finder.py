@@ -704,3 +704,22 @@ def test_passes_exchange_doubles(shape, sigma):
     assert lib.saFilterConvolve(h, img, got) == 0
     lib.saFilterCleanup(h)
     assert numpy.array_equal(got, ref)
+
+
+def test_local_maxima_above_minus_zero():
+    """A threshold of -0.0 is 0.0: zeros and negative values do not exceed it."""
+    from sa_gb300 import ia_utilities_c
+    rng = numpy.random.default_rng(9)
+    img = numpy.round(rng.normal(0.0, 4.0, (40, 65)))
+    img[rng.random(img.shape) < 0.1] = -0.0
+    found = []
+    for threshold in (0.0, -0.0):
+        kw = dict(margin=1, radius=2.0, threshold=threshold, z_range=0, z_values=[0.0])
+        g, o = ia_utilities_c.MaximaFinder(**kw), F.MaximaFinder(**kw)
+        a, b = g.findMaxima([img]), o.findMaxima([img])
+        for u, v in zip(a[:3], b[:3]):
+            assert numpy.array_equal(numpy.asarray(u), numpy.asarray(v))
+        found.append(a[:3])
+        g.cleanup()
+    for u, v in zip(*found):
+        assert numpy.array_equal(numpy.asarray(u), numpy.asarray(v))
