@@ -348,9 +348,13 @@ int saSetPrecision(saFitData *fit, int bits);
 /* Footprint dilation (pixels) used by the dependency scheduler in the first
  * 10 sweeps of a fit (default 3); later sweeps use 0. */
 int saSetDilation(saFitData *fit, int pixels);
-/* At most `ctas` CTAs (4 warps each) for the handle's sweep kernel; 0 (the
- * default) uses the full persistent grid.  A small cap lets the sweeps of
- * several handles run side by side on the device (serving lanes). */
+/* A cap on the handle's sweep grids; 0 (the default) uses the full persistent
+ * grids.  `ctas` counts CTAs that step a peak per warp (4 warps, fewer where
+ * their workspaces do not fit).  Sweeps of four warps a peak take as many
+ * peaks at once, so that many more CTAs; sweeps of eight warps a peak
+ * (splines, FFT PSF, pupil function) take `ctas` CTAs of a peak each.  A small
+ * cap lets the sweeps of several handles run side by side on the device
+ * (serving lanes). */
 int saSetSweepCTAs(saFitData *fit, int ctas);
 /* Use this CUDA stream (cudaStream_t) for all work of the handle. */
 int saSetStream(saFitData *fit, void *stream);
@@ -447,10 +451,15 @@ int saSetSchedule(saFitData *fit, int dil_late, int dil_switch);
  * launches and a host poll per sweep (default 8; 0 never).  The results do
  * not change.  Returns 0, or -1 on error. */
 int saSetTailPeaks(saFitData *fit, int peaks);
-/* No reference counterpart: the CTA count of the persistent sweep grid at
- * full occupancy (SMs x resident CTAs), once the handle has its first
- * image; -1 before.  saSetSweepCTAs caps it. */
+/* No reference counterpart: the CTA count of the persistent sweep grid with a
+ * peak per warp at full occupancy (SMs x resident CTAs), once the handle has
+ * its first image; -1 before.  saSetSweepCTAs caps it. */
 int saGetSweepGrid(saFitData *fit);
+/* No reference counterpart: the sweep grids as they are launched, under the
+ * cap: [CTAs with a peak per warp, warps of such a CTA, CTAs with a peak each
+ * (0: not for this model and ROI), threads of such a CTA].  Returns 0, or -1
+ * before the handle's first image. */
+int saGetSweepShape(saFitData *fit, int32_t *out4);
 
 /* No reference counterpart: the engine's damped solves in checkable form.
  * mFitSolve (multi_fit.c:1839-1883) solves (H + lam diag H) x = b with

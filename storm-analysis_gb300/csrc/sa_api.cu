@@ -419,10 +419,16 @@ struct Engine {
     return 0;
   }
 
-  // CTAs of a sweep launch.
+  // CTAs of a sweep launch.  The cap counts CTAs of a peak per warp; a team
+  // sweep of four warps a peak steps as many peaks at once (a serving lane of
+  // 12 CTAs, one 512 x 512 frame of 3,355 peaks: 77 ms; 238 with 12 teams, 121
+  // with warps), one of eight warps a peak has a team per CTA (a mixed stream
+  // of 96 frames, a quarter of them splines: 1.55 s; 2.0 with four teams per
+  // CTA, whose lanes crowd the others out; 7.6 with warps).
   int grid(bool team) const {
     const int g = team ? shapes.team_grid : shapes.grid;
-    return (sweep_ctas_cap > 0 && sweep_ctas_cap < g) ? sweep_ctas_cap : g;
+    const long long cap = (long long)sweep_ctas_cap * (team && shapes.team_threads <= 128 ? shapes.warps : 1);
+    return (cap > 0 && cap < g) ? (int)cap : g;
   }
 
   // Whether a sweep of this many RUNNING peaks (all frames) runs a peak per
@@ -436,12 +442,13 @@ struct Engine {
   // 8,000 peaks 0.08 / 0.15, 64,000 1.91 / 1.64).  The FP64 engine and the
   // splines are worth a team at any load (fits, ms: 51,000 peaks in FP64
   // 187 / 216, 51,000 spline peaks 303 / 689, 14,400 FFT PSF 346 / 818,
-  // 9,600 pupil function 375 / 1425).
+  // 9,600 pupil function 375 / 1425).  A capped grid has fewer warps to fill
+  // (64 x 512 x 512 3d frames, 3 CTAs per SM: 274 ms, 288 by the full grid).
   bool team_sweep(long long running) const {
     if (shapes.team_grid == 0) return false;
     if (prec == 64 || cfg.model >= M_SPLINE2D) return true;
     const double cover = (double)running * cfg.nroi / ((double)F * npix);
-    return running < 6.0 * shapes.grid * shapes.warps * (1.0 + 0.3 * cover);
+    return running < 6.0 * grid(false) * shapes.warps * (1.0 + 0.3 * cover);
   }
 
   cudaError_t enqueue_sweep(bool team) {
@@ -1663,6 +1670,16 @@ int saGetSweepGrid(saFitData* h) {
   return e->shapes.grid;
 }
 
+int saGetSweepShape(saFitData* h, int32_t* out4) {
+  Engine* e = E(h);
+  if (!e || !e->configured || !out4) return -1;
+  out4[0] = e->grid(false);
+  out4[1] = e->shapes.warps;
+  out4[2] = e->shapes.team_grid > 0 ? e->grid(true) : 0;
+  out4[3] = e->shapes.team_grid > 0 ? e->shapes.team_threads : 0;
+  return 0;
+}
+
 int saSetTailPeaks(saFitData* h, int peaks) {
   Engine* e = E(h);
   if (!e || peaks < 0) return -1;
@@ -2114,7 +2131,11 @@ int saSlotLaunch(saFitData* h, int n_ticks) {
   }
   if (!e->ev_poll) CK(cudaEventCreateWithFlags(&e->ev_poll, cudaEventDisableTiming));
   if (e->start_frames()) return -1;
-  const bool team = e->team_sweep(0);   // a serving grid is small: its lanes share the GPU
+  // Teams whatever the slots hold: a lane's grid is small and other lanes share
+  // the GPU, so a step's time counts (lanes of 1, 8, 32 slots, 256 x 256, ms
+  // with teams / by the RUNNING peaks: 3d 43 57 83 / 53 65 88, 2d 18.8 23.6
+  // 31.3 / 19.3 23.9 31.5, Z 35 54 92 / 45 59 90).
+  const bool team = e->team_sweep(0);
   for (int i = 0; i < n_ticks; i++)
     if (e->tick(team, -1)) return -1;
   CK(cudaMemcpy2DAsync(e->h_ctl, sizeof(FrameCtl), e->d_ctl, sizeof(FrameCtl), offsetof(FrameCtl, escaped), e->F,

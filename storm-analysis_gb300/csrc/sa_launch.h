@@ -25,6 +25,7 @@ struct Shapes {
   int warps = 0;           // warps of such a CTA
   int team_grid = 0;       // the same with a peak per CTA (0: no team step, or no room for one)
   size_t team_smem = 0;
+  int team_threads = 0;
   size_t cta_smem = 0;     // per-frame CTAs
   size_t warp_smem = 0;    // warp-per-peak auxiliary CTAs
 };

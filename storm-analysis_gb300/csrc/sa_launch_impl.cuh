@@ -119,6 +119,7 @@ cudaError_t Launch<T>::configure(const ModelCfg& cfg, Shapes* sh) {
   sh->grid = nsm * (per_sm < 1 ? 1 : per_sm);
   // the team kernels, where a team's workspace fits
   sh->team_smem = k.team_bytes + roi_table_bytes(cfg.nroi);
+  sh->team_threads = k.team_threads;
   if (k.team_sweep && raise_limit((const void*)k.team_sweep, sh->team_smem) == cudaSuccess &&
       raise_limit((const void*)k.team_tail, sh->team_smem) == cudaSuccess) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.team_sweep, k.team_threads, sh->team_smem);

@@ -12,9 +12,10 @@ is rolled back and re-run):
                  escape (and re-run) more often
     dil_late     dilation once most peaks have converged
     dil_switch   the sweep at which the dilation changes
-    ctas_per_sm  resident CTAs (4 peaks each) per SM of the persistent
-                 sweep grid: more overlap of the peaks' latency chains,
-                 more contention
+    ctas_per_sm  resident CTAs per SM of a sweep with a peak per warp (4
+                 peaks each; saSetSweepCTAs says what it means for sweeps
+                 with several warps a peak): more overlap of the peaks'
+                 latency chains, more contention
 
 tune() times complete fits of a sample of the workload's frames for each
 candidate, one parameter at a time (coordinate descent from the default),

@@ -248,6 +248,8 @@ def _declare(lib):
     lib.saSetSchedule.restype = ci
     lib.saGetSweepGrid.argtypes = [hp]
     lib.saGetSweepGrid.restype = ci
+    lib.saGetSweepShape.argtypes = [hp, i32]
+    lib.saGetSweepShape.restype = ci
     lib.saSetTailPeaks.argtypes = [hp, ci]
     lib.saSetTailPeaks.restype = ci
     lib.saSetSweepCTAs.argtypes = [hp, ci]
@@ -347,7 +349,7 @@ EXPORTS = ["daoInitialize", "daoInitialize2DFixed", "daoInitialize2D", "daoIniti
            "saGetPeakPropertyBatch", "saGetPeakPropertyIntBatch", "saSetTiming", "saGetTiming",
            "saGetKernelLaunches", "saGetResultsBatch", "saSetDevice", "saGetSweepTimes",
            "saGetFitImageNoAlloc", "saSlotLoad", "saSlotLaunch", "saSlotPoll", "saSlotReady", "saSlotResults",
-           "saSetSweepCTAs", "saSolveDamped", "saSetSchedule", "saGetSweepGrid", "saSetTailPeaks"]
+           "saSetSweepCTAs", "saSolveDamped", "saSetSchedule", "saGetSweepGrid", "saGetSweepShape", "saSetTailPeaks"]
 
 FINDER_EXPORTS = ["saFilterCreate", "saFilterAnalyze", "saFilterConvolve", "saFilterConvolveMemo", "saFilterCleanup",
                   "saFilterConvolveDevice", "saFilterResultDevice", "saFilterInfo", "saFilterSetStream",

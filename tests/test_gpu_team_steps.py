@@ -125,3 +125,31 @@ def test_rejected_trials_do_not_reach_their_successors(cfg, roi):
         for a, b in zip(first, again):
             assert numpy.array_equal(a, b, equal_nan=True)
     fit.close()
+
+
+@pytest.mark.parametrize("cfg,precision,per_cta", [(1, 32, 4), (2, 32, 4), (0, 64, 4), (3, 32, 1)])
+def test_a_capped_grid_steps_the_same_peaks_at_once(cfg, precision, per_cta):
+    """saSetSweepCTAs counts CTAs of a peak per warp: teams of four warps take
+    as many peaks at once, teams of eight a peak per CTA, none more than the
+    full grid; the results are the uncapped ones."""
+    wl = wild_workload(cfg, 60 + cfg)
+    rows = []
+    full = numpy.zeros(4, dtype=numpy.int32)
+    for ctas in (0, 1, 3, 12, 100000):
+        fit = model_fitter(wl, precision)
+        shape = numpy.zeros(4, dtype=numpy.int32)
+        assert fit.clib.saGetSweepShape(fit.h, shape) == -1   # no image yet
+        assert fit.clib.saSetSweepCTAs(fit.h, ctas) == 0
+        rows.append(fit_rows(fit, wl, 40))
+        assert fit.clib.saGetSweepShape(fit.h, shape) == 0
+        if ctas == 0:
+            full[:] = shape
+            assert full[0] == fit.clib.saGetSweepGrid(fit.h) and full[1] == 4
+            assert full[3] == (128 if per_cta == 4 else 256)
+        else:
+            assert shape[0] == min(ctas, full[0]) and shape[1] == full[1]
+            assert shape[2] == min(ctas * per_cta, full[2]) and shape[3] == full[3]
+        fit.close()
+    for r in rows[1:]:
+        for a, b in zip(rows[0], r):
+            assert numpy.array_equal(a, b, equal_nan=True)
