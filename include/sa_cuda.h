@@ -460,6 +460,11 @@ int saGetSweepGrid(saFitData *fit);
  * (0: not for this model and ROI), threads of such a CTA].  Returns 0, or -1
  * before the handle's first image. */
 int saGetSweepShape(saFitData *fit, int32_t *out4);
+/* No reference counterpart: on = 0 steps every peak by one warp, as ROIs and
+ * pupil functions whose team workspace does not fit an SM are stepped in any
+ * case; 1 (the default) by a CTA where that is faster.  No result depends on
+ * it.  Returns 0, or -1 on error. */
+int saSetTeamSteps(saFitData *fit, int on);
 
 /* No reference counterpart: the engine's damped solves in checkable form.
  * mFitSolve (multi_fit.c:1839-1883) solves (H + lam diag H) x = b with

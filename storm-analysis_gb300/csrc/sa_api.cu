@@ -143,6 +143,7 @@ struct Engine {
   cudaStream_t own_stream = nullptr;   // created for graph capture when no stream was set
   Shapes shapes;
   int sweep_ctas_cap = 0;   // 0: the full persistent grid
+  bool team_steps = true;   // a peak per CTA where that is the faster
   int tail_peaks = 8;       // k_tail for frames with at most this many RUNNING peaks (0: never)
   bool configured = false;
 
@@ -445,7 +446,7 @@ struct Engine {
   // 9,600 pupil function 375 / 1425).  A capped grid has fewer warps to fill
   // (64 x 512 x 512 3d frames, 3 CTAs per SM: 274 ms, 288 by the full grid).
   bool team_sweep(long long running) const {
-    if (shapes.team_grid == 0) return false;
+    if (!team_steps || shapes.team_grid == 0) return false;
     if (prec == 64 || cfg.model >= M_SPLINE2D) return true;
     const double cover = (double)running * cfg.nroi / ((double)F * npix);
     return running < 6.0 * grid(false) * shapes.warps * (1.0 + 0.3 * cover);
@@ -535,8 +536,10 @@ struct Engine {
           else all = false;
         }
         if (all && any) {
-          if (prec == 32) CK(Launch<float>::tail(cfg, fs<float>(), shapes, tail_peaks, stream));
-          else CK(Launch<double>::tail(cfg, fs<double>(), shapes, tail_peaks, stream));
+          Shapes s = shapes;
+          if (!team_steps) s.team_grid = 0;
+          if (prec == 32) CK(Launch<float>::tail(cfg, fs<float>(), s, tail_peaks, stream));
+          else CK(Launch<double>::tail(cfg, fs<double>(), s, tail_peaks, stream));
           launches += 1;
           tail_queued = true;
         }
@@ -1675,8 +1678,16 @@ int saGetSweepShape(saFitData* h, int32_t* out4) {
   if (!e || !e->configured || !out4) return -1;
   out4[0] = e->grid(false);
   out4[1] = e->shapes.warps;
-  out4[2] = e->shapes.team_grid > 0 ? e->grid(true) : 0;
-  out4[3] = e->shapes.team_grid > 0 ? e->shapes.team_threads : 0;
+  const bool team = e->team_steps && e->shapes.team_grid > 0;
+  out4[2] = team ? e->grid(true) : 0;
+  out4[3] = team ? e->shapes.team_threads : 0;
+  return 0;
+}
+
+int saSetTeamSteps(saFitData* h, int on) {
+  Engine* e = E(h);
+  if (!e) return -1;
+  e->team_steps = on != 0;
   return 0;
 }
 

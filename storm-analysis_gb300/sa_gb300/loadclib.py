@@ -250,6 +250,8 @@ def _declare(lib):
     lib.saGetSweepGrid.restype = ci
     lib.saGetSweepShape.argtypes = [hp, i32]
     lib.saGetSweepShape.restype = ci
+    lib.saSetTeamSteps.argtypes = [hp, ci]
+    lib.saSetTeamSteps.restype = ci
     lib.saSetTailPeaks.argtypes = [hp, ci]
     lib.saSetTailPeaks.restype = ci
     lib.saSetSweepCTAs.argtypes = [hp, ci]
@@ -349,7 +351,7 @@ EXPORTS = ["daoInitialize", "daoInitialize2DFixed", "daoInitialize2D", "daoIniti
            "saGetPeakPropertyBatch", "saGetPeakPropertyIntBatch", "saSetTiming", "saGetTiming",
            "saGetKernelLaunches", "saGetResultsBatch", "saSetDevice", "saGetSweepTimes",
            "saGetFitImageNoAlloc", "saSlotLoad", "saSlotLaunch", "saSlotPoll", "saSlotReady", "saSlotResults",
-           "saSetSweepCTAs", "saSolveDamped", "saSetSchedule", "saGetSweepGrid", "saGetSweepShape", "saSetTailPeaks"]
+           "saSetSweepCTAs", "saSolveDamped", "saSetSchedule", "saGetSweepGrid", "saGetSweepShape", "saSetTeamSteps", "saSetTailPeaks"]
 
 FINDER_EXPORTS = ["saFilterCreate", "saFilterAnalyze", "saFilterConvolve", "saFilterConvolveMemo", "saFilterCleanup",
                   "saFilterConvolveDevice", "saFilterResultDevice", "saFilterInfo", "saFilterSetStream",

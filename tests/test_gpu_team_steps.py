@@ -153,3 +153,113 @@ def test_a_capped_grid_steps_the_same_peaks_at_once(cfg, precision, per_cta):
     for r in rows[1:]:
         for a, b in zip(rows[0], r):
             assert numpy.array_equal(a, b, equal_nan=True)
+
+
+def spline2d_workload(knots, nx, ny, n, seed):
+    """Emitters of a measured 2D PSF (the Z model's at focus, knots - 1 px wide)."""
+    from sa_gb300 import synth
+    rng = numpy.random.default_rng(seed)
+    a = numpy.arange(knots) - 0.5 * (knots - 1)
+    coef = rng.normal(0.0, 1.0, 6)
+    samples = synth._aberrated_psf(a[:, None], a[None, :], 0.0, coef)
+    half = 0.5 * (knots - 1)
+    x, y = rng.uniform(half + 2, nx - half - 3, n), rng.uniform(half + 2, ny - half - 3, n)
+    h = rng.uniform(1000.0, 4000.0, n)
+    img = numpy.full((ny, nx), 20.0)
+    for i in range(n):
+        img += h[i] * synth._aberrated_psf(numpy.arange(nx)[None, :] - x[i], numpy.arange(ny)[:, None] - y[i], 0.0, coef)
+    return dict(nx=nx, ny=ny, images=[rng.poisson(img).astype(numpy.float64)], backgrounds=[numpy.full((ny, nx), 20.0)],
+                guesses=[dict(x=x + rng.normal(0.0, 0.3, n), y=y + rng.normal(0.0, 0.3, n), z=numpy.zeros(n),
+                              background=numpy.full(n, 20.0), height=h * rng.uniform(0.8, 1.2, n))],
+                rqe=numpy.ones((ny, nx)), scmos_cal=numpy.zeros((ny, nx)),
+                fitter=dict(model="spline2D", spline=dict(coeff=synth.bicubic_coefficients(samples))))
+
+
+def any_workload(model):
+    from sa_gb300 import psf_fft_c, pupil_fn, synth
+    if model in ("fft", "pupil"):
+        make = synth.fft_workload if model == "fft" else synth.pupil_workload
+        wl = make(frames=2, nx=96, ny=90, n_emitters=25, seed=33, **({} if model == "fft" else dict(size=20)))
+        fk = wl["fitter"]
+        wl["fitter"] = dict(model=model, psf_fft=psf_fft_c.PSFFFT(fk["psf"])) if model == "fft" else dict(
+            model=model, pupil_fn=pupil_fn.PupilFunction(pf_data=fk["pf_data"], zmin=-500.0, zmax=500.0))
+        rng = numpy.random.default_rng(34)
+        for g in wl["guesses"]:
+            g["x"] = numpy.clip(g["x"] + rng.uniform(-3.0, 3.0, 25), 12.0, 84.0)
+            g["y"] = numpy.clip(g["y"] + rng.uniform(-3.0, 3.0, 25), 12.0, 78.0)
+        return wl
+    if model == "spline2D":
+        wl = spline2d_workload(20, 96, 90, 40, 35)
+        wl["guesses"][0]["x"] = numpy.clip(wl["guesses"][0]["x"] + numpy.linspace(-5.0, 5.0, 40), 12.0, 84.0)
+        return wl
+    wl = wild_workload({"2dfixed": 0, "2d": 0, "3d": 1, "Z": 2, "spline3D": 3}[model], 80)
+    wl["fitter"]["model"] = model
+    return wl
+
+
+@pytest.mark.parametrize("model,precision", [("2dfixed", 32), ("2d", 32), ("3d", 32), ("Z", 32), ("spline2D", 32),
+                                             ("spline3D", 32), ("2dfixed", 64), ("2d", 64), ("3d", 64), ("Z", 64),
+                                             ("spline2D", 64), ("spline3D", 64), ("fft", 64), ("pupil", 64)])
+def test_team_and_warp_steps_give_the_same_bits(model, precision):
+    """Every model and engine, from starts that reject trials, leave ROIs and
+    lose peaks: sweeps and tails by teams against sweeps and tails by warps."""
+    wl = any_workload(model)
+    rows = []
+    shape = numpy.zeros(4, dtype=numpy.int32)
+    for on in (1, 0):
+        for tail in (0, 8):
+            fit = model_fitter(wl, precision)
+            assert fit.clib.saSetTeamSteps(fit.h, on) == 0 and fit.clib.saSetTailPeaks(fit.h, tail) == 0
+            rows.append(fit_rows(fit, wl, 150))
+            assert fit.clib.saGetSweepShape(fit.h, shape) == 0 and (shape[2] > 0) == (on == 1)
+            fit.close()
+    assert rows[0][2][1] > 0
+    for r in rows[1:]:
+        for a, b in zip(rows[0], r):
+            assert numpy.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("model,precision,roi", [("2d", 64, 60), ("3d", 64, 60), ("3d", 32, 64), ("spline2D", 32, 62),
+                                                 ("spline2D", 64, 62), ("spline2D", 32, 19), ("spline2D", 64, 19)])
+def test_rois_too_large_for_a_team(model, precision, roi):
+    """ROIs whose team workspace does not fit an SM take a warp per peak; the
+    2D spline at a usual size a team.  Both against the FP64 oracle."""
+    from oracle.oracle import OracleFitter
+    from sa_gb300 import parity, synth
+    if model == "spline2D":
+        wl = spline2d_workload(roi + 1, 150, 140, 12, 41)
+    else:
+        wl = synth.make_workload(0 if model == "2d" else 1, frames=1, nx=150, ny=140, seed=42, n_emitters=12)
+        for k in ("x", "y"):   # inside the larger ROI's margin
+            n = (150 if k == "x" else 140) - roi - 3
+            wl["guesses"][0][k] = roi / 2 + 1 + (wl["guesses"][0][k] - 12.0) * n / ((150 if k == "x" else 140) - 24.0)
+            wl["truth"][0][k] = roi / 2 + 1 + (wl["truth"][0][k] - 12.0) * n / ((150 if k == "x" else 140) - 24.0)
+        t, g = wl["truth"][0], wl["guesses"][0]
+        yy, xx = numpy.mgrid[0:140, 0:150]
+        img = numpy.full((140, 150), g["background"][0])
+        for i in range(12):
+            img += t["height"][i] * numpy.exp(-(xx - t["x"][i]) ** 2 / (2 * g["xsigma"][i] ** 2)
+                                              - (yy - t["y"][i]) ** 2 / (2 * g["ysigma"][i] ** 2))
+        wl["images"][0] = numpy.random.default_rng(43).poisson(img).astype(numpy.float64)
+        wl["fitter"]["roi_size"] = roi
+    kw = dict(wl["fitter"])
+    m = kw.pop("model")
+    if m == "spline2D":
+        kw["spline"] = kw["spline"]["coeff"]
+    ref = OracleFitter(m, (140, 150), **kw)
+    ref.newImage(wl["images"][0])
+    ref.newBackground(wl["backgrounds"][0])
+    ref.newPeaks(wl["guesses"][0], "hdf5")
+    ref.doFit(100)
+    props = ("x", "y", "z", "height", "background", "status", "iterations")
+    want = {p: ref.getPeakProperty(p) for p in props}
+    ref.cleanup()
+    assert (want["status"] == 1).sum() >= 8
+    fit = model_fitter(wl, precision)
+    fit.load(numpy.stack(wl["images"]), numpy.stack(wl["backgrounds"]), wl["guesses"], "hdf5")
+    shape = numpy.zeros(4, dtype=numpy.int32)
+    assert fit.clib.saGetSweepShape(fit.h, shape) == 0 and (shape[2] > 0) == (roi == 19), shape
+    fit.fit(100)
+    st = parity.compare(fit.results(), want)
+    fit.close()
+    assert parity.within_tolerance(st, min_fraction=0.999), st
