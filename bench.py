@@ -1027,7 +1027,7 @@ def run_mp_report(args, pool):
         walls.append(time.perf_counter() - t0)
     f.cleanup(verbose=False)
     cpu_s, ref = pool.map(_mp_cpu_job, [(wl, "liboracle_timing.so")])[0]
-    # batched: MP_FRAMES frames at once (one warp each) against the oracle's
+    # batched: MP_FRAMES frames at once against the oracle's
     # frames on the host cores (one frame per process)
     # 64 distinct frames, repeated to MP_FRAMES (the content of a frame does
     # not depend on its neighbours in the batch)
